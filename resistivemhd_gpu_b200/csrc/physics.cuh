@@ -48,6 +48,27 @@ template <typename T> __device__ __forceinline__ T minmod(T x, T y, T eps)
     return x > T(0) ? m : (x < T(0) ? -m : T(0) * m);
 }
 
+
+__host__ __device__ __forceinline__ unsigned int hi_word(double x)
+{
+#ifdef __CUDA_ARCH__
+    return (unsigned int)__double2hiint(x);
+#else
+    unsigned long long u;
+    memcpy(&u, &x, sizeof(u));
+    return (unsigned int)(u >> 32);
+#endif
+}
+__host__ __device__ __forceinline__ unsigned int lo_word(double x)
+{
+#ifdef __CUDA_ARCH__
+    return (unsigned int)__double2loint(x);
+#else
+    unsigned long long u;
+    memcpy(&u, &x, sizeof(u));
+    return (unsigned int)u;
+#endif
+}
 // Single-precision reciprocal and square roots of the FP32-bulk variant
 // (hardware approximations, ~1 ulp of float).  A host build of the kernels
 // (CPU tests, RMHD_HOST_EMULATION) takes the correctly rounded values.
@@ -154,38 +175,21 @@ __device__ __forceinline__ double rcp_rn_md(double b)
     return fma(y, e, y);
 }
 
-__host__ __device__ __forceinline__ unsigned int hi_word(double x)
-{
-#ifdef __CUDA_ARCH__
-    return (unsigned int)__double2hiint(x);
-#else
-    unsigned long long u;
-    memcpy(&u, &x, sizeof(u));
-    return (unsigned int)(u >> 32);
-#endif
-}
-__host__ __device__ __forceinline__ unsigned int lo_word(double x)
-{
-#ifdef __CUDA_ARCH__
-    return (unsigned int)__double2loint(x);
-#else
-    unsigned long long u;
-    memcpy(&u, &x, sizeof(u));
-    return (unsigned int)u;
-#endif
-}
-
 // Division policy of the exact arithmetic: shared reciprocals with the
 // guard above.  recip(b) returns y; div(a, b, y) returns RN(a/b) whenever ok
-// stays true.
-struct MdDiv {
+// stays true.  BTOP and QTOP are the exponents that divisors and quotients
+// have to stay below (at most 400 and 500 for the theorem's conditions).
+// The range tests work on twice the high word, which drops the sign.
+template <int BTOP, int QTOP> struct MdDivT {
+    static_assert(BTOP <= 400 && QTOP <= 500, "ranges in which the correction rounds correctly");
     bool ok = true;
     __device__ __forceinline__ double recip(double b)
     {
         const unsigned int h = hi_word(b);
-        // |b| in [2^-400, 2^400): biased exponent in [623, 1423)
-        ok &= ((h & 0x7FFFFFFFu) - 0x26F00000u) < 0x32000000u;
-        ok &= ((h & 0x000FFFFFu) != 0x000FFFFFu) | (lo_word(b) != 0xFFFFFFFFu);
+        // |b| in [2^-400, 2^BTOP): biased exponent in [623, 1023 + BTOP)
+        ok &= (h * 2u - (623u << 21)) < ((400u + BTOP) << 21);
+        // not an all-ones significand
+        ok &= ((~h & 0x000FFFFFu) | ~lo_word(b)) != 0u;
         return rcp_rn_md(b);
     }
     __device__ __forceinline__ double div(double a, double b, double y)
@@ -194,11 +198,15 @@ struct MdDiv {
         const double r = fma(-q, b, a);
         const double q1 = fma(r, y, q);
         const bool z = a == 0.0;
-        // |q| in [2^-500, 2^500): biased exponent in [523, 1523)
-        ok &= z | (((hi_word(q) & 0x7FFFFFFFu) - 0x20B00000u) < 0x3E800000u);
+        // |q| in [2^-500, 2^QTOP): biased exponent in [523, 1023 + QTOP)
+        ok &= z | ((hi_word(q) * 2u - (523u << 21)) < ((500u + QTOP) << 21));
         return z ? q : q1;
     }
 };
+using MdDiv = MdDivT<400, 500>;
+// The HLLD flux's own: with every divisor and quotient below 2^240 (and the
+// velocities bounded, hlld_flux_sel), no candidate flux can overflow.
+using MdDivFlux = MdDivT<240, 240>;
 
 // Division policy with plain IEEE division (the fallback of MdDiv).
 struct IeeeDiv {
@@ -443,21 +451,35 @@ __device__ __forceinline__ void hlld_flux_ieee(const Prim &L, const Prim &R, dou
 // candidate states (38 values) live until the region flags are known and
 // then selects; here each candidate is taken into the nine `c*` values as
 // soon as its own flag is known, so the left and right input states die
-// after the star states, and the magnitude guard is summed as the values
-// appear.  Where the shortcut's conditions fail -- a guard of the shared
-// reciprocals, more or fewer than one region selected, a value of 1e75 or
-// more (or non-finite) -- it returns false with f unwritten, and the caller
-// forms the interface with hlld_flux_ieee, away from its common path (the
-// stage kernel's flux phase does that after its loop, for the interfaces
-// that asked, so the rare path does not shape the common path's registers).
+// after the star states.  Where the shortcut's conditions fail it returns
+// false with f unwritten, and the caller forms the interface with
+// hlld_flux_ieee, away from its common path (the stage kernel's flux phase
+// does that after its loop, for the interfaces that asked, so the rare path
+// does not shape the common path's registers).  The conditions:
+//
+// 1. dv.ok: every divisor and quotient is finite and below 2^240.
+// 2. The six velocities are below 1e71.  With 1, the densities (divisors),
+//    |B| (|B|^2 / rho is a quotient), p (p / (gm - 1) is one), SM, pT1 and
+//    the star states are bounded too: v1 and w1 differ from v and w by a
+//    quotient, e2 from e1 by sqrt(rho1) times products of two such values.
+//    No candidate flux, a product of at most three of these (or of e2 and
+//    one), reaches 2^1024, so the reference's F * 0 of the five others is
+//    +-0 and leaves the selected flux bit for bit.
+// 3. Exactly one region.  SL <= 0 after its clamp, so the left outer state
+//    is never selected.  Under 1, SM, S1L, S1R and SR are not NaN (rho1 < 0
+//    makes sqL + sqR NaN, a divisor) and S1L <= SM <= S1R, since each adds
+//    or subtracts a root; then 0 falls in exactly one of the regions ML, IL,
+//    IR, and right of S1R; the last is MR for SR > 0, else OR.  SR = 0 with
+//    S1R > 0 selects OR and one more: declined.
 __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, double gm, double EPS, double ygm1,
                                               bool gm1_ok, double f[8])
 {
-    MdDiv dv;
+    MdDivFlux dv;
     dv.ok = gm1_ok;
     const double rhoL = L.rho, uL = L.u, vL = L.v, wL = L.w, bXL = L.bX, bYL = L.bY, bZL = L.bZ, pL = L.p;
     const double rhoR = R.rho, uR = R.u, vR = R.v, wR = R.w, bXR = R.bX, bYR = R.bY, bZR = R.bZ, pR = R.p;
     const double gm1 = gm - 1.0;
+    dv.ok &= (fabs(uL) + fabs(vL) + fabs(wL)) + (fabs(uR) + fabs(vR) + fabs(wR)) < 1e71;
 
     const double eL = dv.div(pL, gm1, ygm1)
                     + 0.5 * rhoL * (uL * uL + vL * vL + wL * wL)
@@ -467,11 +489,6 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
                     + 0.5 * rhoR * (uR * uR + vR * vR + wR * wR)
                     + 0.5 * (bXR * bXR + bYR * bYR + bZR * bZR);
     const double pTR = pR + 0.5 * (bXR * bXR + bYR * bYR + bZR * bZR);
-    // magnitude guard of the shortcut (any order of summation will do: the
-    // guard only chooses between two evaluations with the same bits)
-    double mag = fabs(rhoL) + fabs(uL) + fabs(vL) + fabs(wL) + fabs(bXL) + fabs(bYL) + fabs(bZL) + fabs(eL)
-               + fabs(pTL) + fabs(rhoR) + fabs(uR) + fabs(vR) + fabs(wR) + fabs(bXR) + fabs(bYR) + fabs(bZR)
-               + fabs(eR) + fabs(pTR);
 
     const double yrL = dv.recip(rhoL), yrR = dv.recip(rhoR);
     const double csL = sqrt(dv.div(gm * pL, rhoL, yrL));
@@ -492,20 +509,17 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
     SL = tmin(SL, 0.0);
     SR = tmax(SR, 0.0);
 
-    // the outer states: candidates of their own
-    const bool bOL = SL > 0.0;
-    const bool bOR = SR <= 0.0;
-    double cr = bOL ? rhoL : rhoR, cu = bOL ? uL : uR, cv = bOL ? vL : vR, cw = bOL ? wL : wR;
-    double cbx = bOL ? bXL : bXR, cby = bOL ? bYL : bYR, cbz = bOL ? bZL : bZR;
-    double ce = bOL ? eL : eR, cpt = bOL ? pTL : pTR;
-    int nsel = (int)bOL + (int)bOR;
+    // the right outer state, a candidate of its own
+    const bool rgt = 0.0 < SR;   // not OR
+    double cr = rhoR, cv = vR, cw = wR, cbx = bXR, cby = bYR, cbz = bZR, ce = eR;
 
     const double den = (SR - uR) * rhoR - (SL - uL) * rhoL + EPS;
     const double yden = dv.recip(den);
     const double SM = dv.div((SR - uR) * rhoR * uR - (SL - uL) * rhoL * uL - pTR + pTL, den, yden);
     const double pT1 = dv.div((SR - uR) * rhoR * pTL - (SL - uL) * rhoL * pTR
                               + rhoL * rhoR * (SR - uR) * (SL - uL) * (uR - uL), den, yden);
-    mag += fabs(SM) + fabs(pT1);
+    // the velocity and total pressure of every state inside the fan
+    const double cu = rgt ? SM : uR, cpt = rgt ? pT1 : pTR;
 
     // left star state (u1L = SM, bX1L = bXL)
     const double dLM = SL - SM + EPS;
@@ -522,13 +536,11 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
     const double e1L = dv.div((SL - uL) * eL - pTL * uL + pT1 * SM
                               + bXL * ((uL * bXL + vL * bYL + wL * bZL) - vb1L),
                               dLM, yLM);
-    mag += fabs(rho1L) + fabs(v1L) + fabs(w1L) + fabs(bY1L) + fabs(bZ1L) + fabs(e1L);
     const double yr1L = dv.recip(rho1L);
     const double S1L = SM - sqrt(dv.div(bXL * bXL, rho1L, yr1L));
-    const bool bML = (SL <= 0.0) && (0.0 < S1L);
-    const bool bIL = (S1L <= 0.0) && (0.0 < SM);
+    const bool bML = 0.0 < S1L;
     if (bML) {
-        cr = rho1L; cu = SM; cv = v1L; cw = w1L; cbx = bXL; cby = bY1L; cbz = bZ1L; ce = e1L; cpt = pT1;
+        cr = rho1L; cv = v1L; cw = w1L; cbx = bXL; cby = bY1L; cbz = bZ1L; ce = e1L;
     }
 
     // right star state
@@ -546,17 +558,15 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
     const double e1R = dv.div((SR - uR) * eR - pTR * uR + pT1 * SM
                               + bXR * ((uR * bXR + vR * bYR + wR * bZR) - vb1R),
                               dRM, yRM);
-    mag += fabs(rho1R) + fabs(v1R) + fabs(w1R) + fabs(bY1R) + fabs(bZ1R) + fabs(e1R);
     const double yr1R = dv.recip(rho1R);
     const double S1R = SM + sqrt(dv.div(bXR * bXR, rho1R, yr1R));
-    const bool bMR = (S1R <= 0.0) && (0.0 < SR);
-    const bool bIR = (SM <= 0.0) && (0.0 < S1R);
-    if (bMR) {
-        cr = rho1R; cu = SM; cv = v1R; cw = w1R; cbx = bXR; cby = bY1R; cbz = bZ1R; ce = e1R; cpt = pT1;
+    const bool in1R = 0.0 < S1R;   // left of the right Alfven wave
+    if (rgt & !in1R) {             // MR
+        cr = rho1R; cv = v1R; cw = w1R; cbx = bXR; cby = bY1R; cbz = bZ1R; ce = e1R;
     }
-    nsel += (int)bML + (int)bIL + (int)bMR + (int)bIR;
 
     // double-star states (u2 = SM)
+    const bool bIL = !bML & (0.0 < SM), bI = !bML & in1R;   // IL; IL or IR
     const double sqL = sqrt(rho1L), sqR = sqrt(rho1R), sqLR = sqrt(rho1L * rho1R);
     const double sbX = sgn(bXL);
     const double dsq = sqL + sqR + EPS;
@@ -567,13 +577,12 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
     const double bZ2 = dv.div(sqL * bZ1R + sqR * bZ1L + sqLR * (w1R - w1L) * sbX, dsq, ysq);
     const double e2L = e1L - sqL * (vb1L - (SM * bXL + v2 * bY2 + w2 * bZ2)) * sgn(bXL);
     const double e2R = e1R + sqR * (vb1R - (SM * bXR + v2 * bY2 + w2 * bZ2)) * sgn(bXR);
-    mag += fabs(v2) + fabs(w2) + fabs(bY2) + fabs(bZ2) + fabs(e2L) + fabs(e2R);
-    if (bIL | bIR) {
-        cr = bIL ? rho1L : rho1R; cu = SM; cv = v2; cw = w2; cbx = bIL ? bXL : bXR;
-        cby = bY2; cbz = bZ2; ce = bIL ? e2L : e2R; cpt = pT1;
+    if (bI) {
+        cr = bIL ? rho1L : rho1R; cv = v2; cw = w2; cbx = bIL ? bXL : bXR;
+        cby = bY2; cbz = bZ2; ce = bIL ? e2L : e2R;
     }
 
-    if (!dv.ok || nsel != 1 || !(mag < 1e75)) return false;
+    if (!dv.ok | (!rgt & in1R)) return false;
 #pragma unroll
     for (int n = 0; n < 8; ++n) f[n] = 0.0;
     add_one_flux(cr, cu, cv, cw, cbx, cby, cbz, ce, cpt, f);
@@ -588,11 +597,13 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
 // squares their square roots), sqrt(rho*) and |bX|/sqrt(rho*) from one rsqrt,
 // and bX taken once (left and right states share the interface-normal B).
 //
-// ONE = true forms the common case only: exactly one region selected and
-// finite wave speeds.  That region's state is taken into the `c*` values as
+// ONE = true forms the common case only: exactly one region selected and no
+// NaN wave speed.  That region's state is taken into the `c*` values as
 // soon as its flag is known, so the input states need not stay live until
 // the end; it returns false (f unwritten) when the case does not apply.
-// ONE = false forms every case.
+// SL <= 0 after its clamp, S1L <= SM <= S1R (false if either is NaN, as they
+// are when SL, SR or SM is), and so exactly one region holds unless SR = 0
+// and S1R > 0 (see hlld_flux_sel).  ONE = false forms every case.
 template <bool ONE, typename T>
 __device__ __forceinline__ bool hlld_fast_body(const PrimT<T> &L, const PrimT<T> &R, T gm, T inv_gm1, T EPS, T f[8])
 {
@@ -631,10 +642,10 @@ __device__ __forceinline__ bool hlld_fast_body(const PrimT<T> &L, const PrimT<T>
 
     const bool bOL = SL > T(0);
     const bool bOR = SR <= T(0);
-    T cr, cu, cv, cw, cby, cbz, ce, cpt;   // the selected candidate (ONE)
+    const bool rgt = T(0) < SR;
+    T cr, cv, cw, cby, cbz, ce;   // the selected candidate (ONE)
     if (ONE) {
-        cr = bOL ? L.rho : R.rho; cu = bOL ? L.u : R.u; cv = bOL ? L.v : R.v; cw = bOL ? L.w : R.w;
-        cby = bOL ? L.bY : R.bY; cbz = bOL ? L.bZ : R.bZ; ce = bOL ? eL : eR; cpt = bOL ? pTL : pTR;
+        cr = R.rho; cv = R.v; cw = R.w; cby = R.bY; cbz = R.bZ; ce = eR;
     }
 
     const T dSL = SL - uL, dSR = SR - uR;
@@ -666,9 +677,12 @@ __device__ __forceinline__ bool hlld_fast_body(const PrimT<T> &L, const PrimT<T>
     const bool bIL = (S1L <= T(0)) && (T(0) < SM);
     const bool bMR = (S1R <= T(0)) && (T(0) < SR);
     const bool bIR = (SM <= T(0)) && (T(0) < S1R);
-    if (ONE && (bML | bMR)) {
-        cr = bML ? rho1L : rho1R; cu = SM; cv = bML ? v1L : v1R; cw = bML ? w1L : w1R;
-        cby = bML ? bY1L : bY1R; cbz = bML ? bZ1L : bZ1R; ce = bML ? e1L : e1R; cpt = pT1;
+    const bool ml = T(0) < S1L, in1R = T(0) < S1R;
+    if (ONE && ml) {
+        cr = rho1L; cv = v1L; cw = w1L; cby = bY1L; cbz = bZ1L; ce = e1L;
+    }
+    if (ONE && (rgt & !in1R)) {
+        cr = rho1R; cv = v1R; cw = w1R; cby = bY1R; cbz = bZ1R; ce = e1R;
     }
     const T sb = sgn(bX);
     const T id2 = rcp_nr(sqL + sqR + EPS);
@@ -684,14 +698,14 @@ __device__ __forceinline__ bool hlld_fast_body(const PrimT<T> &L, const PrimT<T>
     const int nsel = (int)bOL + (int)bML + (int)bIL + (int)bOR + (int)bMR + (int)bIR;
     const bool nan_speed = (SL != SL) | (SR != SR) | (SM != SM) | (S1L != S1L) | (S1R != S1R);
     if (ONE) {
-        if (nsel != 1 || nan_speed) return false;
-        if (bIL | bIR) {
-            cr = bIL ? rho1L : rho1R; cu = SM; cv = v2; cw = w2; cby = bY2; cbz = bZ2; ce = bIL ? e2L : e2R;
-            cpt = pT1;
+        if (!(S1L <= S1R) | (!rgt & in1R)) return false;
+        const bool il = T(0) < SM;
+        if (!ml & in1R) {
+            cr = il ? rho1L : rho1R; cv = v2; cw = w2; cby = bY2; cbz = bZ2; ce = il ? e2L : e2R;
         }
 #pragma unroll
         for (int n = 0; n < 8; ++n) f[n] = T(0);
-        add_one_flux(cr, cu, cv, cw, bX, cby, cbz, ce, cpt, f);
+        add_one_flux(cr, rgt ? SM : uR, cv, cw, bX, cby, cbz, ce, rgt ? pT1 : pTR, f);
         return true;
     }
 #pragma unroll
