@@ -47,6 +47,10 @@ struct rmhd2d_solver {
     double *row2 = nullptr;      // nx doubles
     Control *ctl = nullptr;      // device control block
     Control *ctl_host = nullptr; // pinned mirror for readback
+    // The last work enqueued that changes the control block was a one-step
+    // graph, which leaves the control block in ctl_host itself.
+    bool mirrored = false;
+    bool captured = false;       // a caller has captured a step: its replays change the control block unseen
     // per tile shape: stage-1 source A, stage-2 source B, eta plane with the
     // stage-1 and stage-2 boxes
     CUtensorMap mapA[NSHAPE]{}, mapB[NSHAPE]{}, mapE1[NSHAPE]{}, mapE2[NSHAPE]{};
@@ -160,7 +164,8 @@ bool encode_eta_map(CUtensorMap *map, const Grid &g, double *base, int ui, int u
 int sync_and_check(rmhd2d_solver *s)
 {
     // The control block is read behind the stream's work: one wait covers both.
-    CK(cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s->stream));
+    if (!s->mirrored)
+        CK(cudaMemcpyAsync(s->ctl_host, s->ctl, sizeof(Control), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     if (s->ctl_host->error != KERR_NONE)
         return fail(s, RMHD2D_ERR_KERNEL, "a stage kernel's bounded wait for its staged tile expired");
@@ -171,6 +176,7 @@ int sync_and_check(rmhd2d_solver *s)
 // `parity` (after a state change outside a step).
 int refresh_rate(rmhd2d_solver *s)
 {
+    s->mirrored = false;
     CK(cudaMemsetAsync(&s->ctl->amax[s->parity], 0, sizeof(unsigned long long), s->stream));
     CK(cudaMemsetAsync(&s->ctl->first_nan[s->parity], 0, sizeof(int), s->stream));
     CK(cudaMemsetAsync(&s->ctl->crashed, 0, sizeof(int), s->stream));
@@ -228,6 +234,7 @@ BatchLauncher batch_launcher(int precision)
 void enqueue_step_between(rmhd2d_solver *s, int parity, const double *un, const CUtensorMap *map_un, double *ustar,
                           const CUtensorMap *map_ustar, double *dst, double *dt_log, const double *dt_in)
 {
+    s->mirrored = false;
     StageArgs a{};
     a.dt_in = dt_in;
     a.g = s->g;
@@ -252,9 +259,12 @@ void enqueue_step_between(rmhd2d_solver *s, int parity, const double *un, const 
 
 // dt_log: stage 1 also writes the step's dt there (a recorded run); dt_in:
 // the step reads its dt from there (a replayed run).  Not for CT-Contact,
-// whose pipeline takes its dt from the control block.
-void enqueue_step(rmhd2d_solver *s, int parity, double *dt_log = nullptr, const double *dt_in = nullptr)
+// whose pipeline takes its dt from the control block.  mirror: the step ends
+// with the control block copied there.
+void enqueue_step(rmhd2d_solver *s, int parity, double *dt_log = nullptr, const double *dt_in = nullptr,
+                  Control *mirror = nullptr)
 {
+    s->mirrored = false;
     if (s->contact) {
         const size_t P = (size_t)s->g.plane;
         ContactStep c{};
@@ -297,7 +307,7 @@ void enqueue_step(rmhd2d_solver *s, int parity, double *dt_log = nullptr, const 
     a.un = s->A;
     a.dst = s->A;
     launch(2, s->shape2, &s->mapB[s->shape2], &s->mapE2[s->shape2], a, s->stream);
-    launch_boundary(s->g, s->A, s->row2, s->ctl, parity ^ 1, s->stream);
+    launch_boundary_mirrored(s->g, s->A, s->row2, s->ctl, parity ^ 1, mirror, s->stream);
 }
 
 int upload_from_device_aos(rmhd2d_solver *s, const double *aos_dev, int apply_boundary)
@@ -333,6 +343,7 @@ void free_adjoint(AdjointWork *w)
 // Sets or clears Control::use_fixed_dt in stream order.
 int set_fixed_dt_mode(rmhd2d_solver *s, int on)
 {
+    s->mirrored = false;
     static const int kOn = 1, kOff = 0;
     CK(cudaMemcpyAsync(&s->ctl->use_fixed_dt, on ? &kOn : &kOff, sizeof(int), cudaMemcpyHostToDevice, s->stream));
     return RMHD2D_OK;
@@ -643,7 +654,9 @@ static int capture_steps(rmhd2d_solver *s, int parity, int nsteps, cudaGraphExec
 {
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    for (int n = 0; n < nsteps; ++n) enqueue_step(s, parity ^ (n & 1));
+    // a one-step graph ends with the control block in the host's mirror
+    for (int n = 0; n < nsteps; ++n)
+        enqueue_step(s, parity ^ (n & 1), nullptr, nullptr, nsteps == 1 ? s->ctl_host : nullptr);
     cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
     if (e != cudaSuccess) return fail(s, RMHD2D_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     e = cudaGraphInstantiate(ge, graph, 0);
@@ -683,12 +696,15 @@ int rmhd2d_step_rk2(rmhd2d_solver *s)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s->stream, &cap));
     if (cap != cudaStreamCaptureStatusNone) {
+        s->captured = true;
         enqueue_step(s, s->parity);
         CK(cudaGetLastError());
     } else {
         const int rc = ensure_step_graphs(s, s->graph1, 1);
         if (rc) return rc;
+        s->mirrored = false;
         CK(cudaGraphLaunch(s->graph1[s->parity], s->stream));
+        s->mirrored = !s->contact && !s->captured;
     }
     s->parity ^= 1;
     s->steps += 1;
@@ -708,6 +724,7 @@ int rmhd2d_run(rmhd2d_solver *s, int nsteps)
         if (rc) return rc;
     }
     while (nsteps >= 2) {
+        s->mirrored = false;
         CK(cudaGraphLaunch(s->graph2[s->parity], s->stream));
         s->steps += 2;
         nsteps -= 2;
@@ -748,6 +765,7 @@ int rmhd2d_profile_step(rmhd2d_solver *s, float *ms4)
         ev[n] = sev[n].e;
     }
     const int parity = s->parity;
+    s->mirrored = false;
     StageArgs a{};
     a.g = s->g;
     a.eta = s->eta;
@@ -924,6 +942,7 @@ static int snapshot_take(rmhd2d_solver *s, Snapshot &sn)
 static int snapshot_restore(rmhd2d_solver *s, Snapshot &sn)
 {
     const size_t bytes = (size_t)s->g.plane * NFIELD * sizeof(double);
+    s->mirrored = false;
     CK(cudaMemcpyAsync(s->A, sn.A, bytes, cudaMemcpyDeviceToDevice, s->stream));
     CK(cudaMemcpyAsync(s->ctl, &sn.ctl, sizeof(Control), cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
@@ -1482,6 +1501,7 @@ int rmhd2d_slab_stage(rmhd2d_solver *s, int stage)
     if (stage != 1 && stage != 2) return fail(s, RMHD2D_ERR_INVALID, "stage must be 1 or 2");
     if (!s->has_state) return fail(s, RMHD2D_ERR_STATE, "no state set");
     CK(cudaSetDevice(s->device));
+    s->mirrored = false;
     StageArgs a{};
     a.g = s->g;
     a.eta = s->eta;
@@ -1511,6 +1531,7 @@ int rmhd2d_slab_fill(rmhd2d_solver *s, int which)
     if (which < 0 || which > 2) return fail(s, RMHD2D_ERR_INVALID, "which must be 0, 1 or 2");
     if (!s->has_state) return fail(s, RMHD2D_ERR_STATE, "no state set");
     CK(cudaSetDevice(s->device));
+    s->mirrored = false;
     if (which == 0) {
         if (s->g.bc_x == BC_SYMMETRIC) launch_snapshot_row2(s->g, s->A, s->row2, s->stream);
         launch_boundary(s->g, s->A, s->row2, nullptr, 0, s->stream);
@@ -1541,6 +1562,7 @@ int rmhd2d_slab_get_words(rmhd2d_solver *s, long long *dev_words)
     CK(cudaSetDevice(s->device));
     // the domain's ghost column 0 of a periodic-x decomposition sits in the
     // first slab's low halo, which its neighbour has just filled
+    s->mirrored = false;
     if ((s->slab & RMHD2D_SLAB_ORIGIN) && (s->g.x_halo & 1))
         launch_slab_origin_column(s->g, s->A, s->ctl, s->parity, s->stream);
     launch_slab_words(s->ctl, s->parity, dev_words, 1, s->stream);
@@ -1553,6 +1575,7 @@ int rmhd2d_slab_set_words(rmhd2d_solver *s, const long long *dev_words)
     if (!s || !dev_words) return fail(s, RMHD2D_ERR_INVALID, "null argument");
     if (!(s->slab & SLAB_CREATED)) return fail(s, RMHD2D_ERR_STATE, "not a slab (rmhd2d_create_slab)");
     CK(cudaSetDevice(s->device));
+    s->mirrored = false;
     launch_slab_words(s->ctl, s->parity, const_cast<long long *>(dev_words), 0, s->stream);
     CK(cudaGetLastError());
     return RMHD2D_OK;

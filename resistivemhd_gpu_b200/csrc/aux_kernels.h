@@ -9,6 +9,9 @@
 namespace rmhd2d {
 
 void launch_boundary(const Grid &g, double *s, const double *row2, Control *ctl, int slot, cudaStream_t st);
+// The same; the launch then leaves the control block in *mirror (host memory).
+void launch_boundary_mirrored(const Grid &g, double *s, const double *row2, Control *ctl, int slot, Control *mirror,
+                              cudaStream_t st);
 void launch_boundary_batch(const BatchRun *runs, int nruns, long long max_ghost, int which, int slot, cudaStream_t st);
 void launch_snapshot_row2(const Grid &g, const double *s, double *row2, cudaStream_t st);
 void launch_rate(const Grid &g, const double *s, Control *ctl, int slot, int set_crash, cudaStream_t st);

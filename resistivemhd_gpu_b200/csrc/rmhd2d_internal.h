@@ -41,6 +41,7 @@ struct Control {
     int error;                   // kernel-side error code (bounded wait expired, ...)
     double dt_fixed;             // dt of the next step when use_fixed_dt is set
     int use_fixed_dt;            // 1: steps take dt_fixed instead of the CFL dt (frozen-dt runs)
+    unsigned long long ghost_blocks;  // blocks of the step's last ghost fill that have finished (back to 0 after it)
 };
 
 enum KernelError { KERR_NONE = 0, KERR_TMA_TIMEOUT = 1 };
