@@ -53,9 +53,10 @@ struct rmhd2d_solver {
     bool captured = false;       // a caller has captured a step: its replays change the control block unseen
     // per tile shape: stage-1 source A, stage-2 source B, eta plane with the
     // stage-1 and stage-2 boxes
-    CUtensorMap mapA[NSHAPE]{}, mapB[NSHAPE]{}, mapE1[NSHAPE]{}, mapE2[NSHAPE]{};
+    CUtensorMap mapA[NSHAPE_ALL]{}, mapB[NSHAPE_ALL]{}, mapE1[NSHAPE_ALL]{}, mapE2[NSHAPE_ALL]{};
     int shape = 0;                       // tile shape of stage 1
     int shape2 = 0;                      // tile shape of stage 2
+    int own[2] = {-1, -1};               // shape the library picked for a stage (default_shapes, autotune), or -1
     void *batch = nullptr;               // owning batch, if any
     int parity = 0;
     bool has_state = false;
@@ -228,6 +229,46 @@ BatchLauncher batch_launcher(int precision)
     }
 }
 
+// The tile shape a stage runs: the library's own choice until the caller sets
+// one.
+int stage_plan(const rmhd2d_solver *s, int stage)
+{
+    return s->own[stage - 1] >= 0 ? s->own[stage - 1] : stage == 1 ? s->shape : s->shape2;
+}
+
+// Whether a grid's 4 x 16 tiles all run at once, two per SM.  Then a stage
+// lasts one block's latency, and a block of one interface per thread is the
+// fastest: per step at 128 x 128, exact 30.5 -> 22.6 us, fast 23.9 -> 19.5,
+// FP32-bulk 20.6 -> 18.5 against shape 0.  With more tiles a second wave
+// follows, and it loses (160 x 160: 30.8 -> 33.8, 23.8 -> 27.7, 20.5 -> 26.7).
+bool small_grid(const Grid &g)
+{
+    const long long ti = stage_ti(1, SHAPE_SMALL), tj = shape_tj(SHAPE_SMALL);
+    return ((g.nx - 2 * HALO + ti - 1) / ti) * ((g.ny - 2 * HALO + tj - 1) / tj) <= 2 * SM_COUNT;
+}
+
+// The shapes a solver starts with.  Large grids take what the autotuner finds
+// on them: three CTAs per SM win from about 2^18 cells (512 x 512, per step:
+// exact 117.2 -> 111.7 us, fast 84.1 -> 80.2, FP32-bulk 69.6 -> 62.5; 601 x
+// 347 and 384 x 384 are level), below that shape 0.
+void default_shapes(rmhd2d_solver *s)
+{
+    const Grid &g = s->g;
+    if (small_grid(g)) {
+        s->own[0] = s->own[1] = SHAPE_SMALL;
+    } else if ((long long)(g.nx - 2 * HALO) * (g.ny - 2 * HALO) >= 1LL << 18) {
+        s->own[0] = 4;
+        s->own[1] = s->cfg.precision == RMHD2D_FP32_BULK ? 4 : 5;
+    }
+}
+
+// Launches a stage of the solver's plan, reading the state through `map`.
+void launch_planned(rmhd2d_solver *s, int stage, const CUtensorMap *map, const StageArgs &a)
+{
+    const int k = stage_plan(s, stage);
+    stage_launcher(s->cfg.precision)(stage, k, map, stage == 1 ? &s->mapE1[k] : &s->mapE2[k], a, s->stream);
+}
+
 // One stage-1-EMF step from `un` (read through map_un) into `dst`, with U*
 // in `ustar` (read through map_ustar); the same launches as enqueue_step
 // without A and B.  dst may not be un.
@@ -242,18 +283,17 @@ void enqueue_step_between(rmhd2d_solver *s, int parity, const double *un, const 
     a.row2 = s->g.bc_x == BC_SYMMETRIC ? s->row2 : nullptr;
     a.ctl = s->ctl;
     a.parity = parity;
-    auto launch = stage_launcher(s->cfg.precision);
     a.src = un;
     a.un = un;
     a.dst = ustar;
     a.dt_log = dt_log;
-    launch(1, s->shape, map_un, &s->mapE1[s->shape], a, s->stream);
+    launch_planned(s, 1, map_un, a);
     a.dt_log = nullptr;
     launch_boundary(s->g, ustar, s->row2, nullptr, 0, s->stream);
     a.src = ustar;
     a.un = un;
     a.dst = dst;
-    launch(2, s->shape2, map_ustar, &s->mapE2[s->shape2], a, s->stream);
+    launch_planned(s, 2, map_ustar, a);
     launch_boundary(s->g, dst, s->row2, s->ctl, parity ^ 1, s->stream);
 }
 
@@ -293,20 +333,19 @@ void enqueue_step(rmhd2d_solver *s, int parity, double *dt_log = nullptr, const 
     a.ctl = s->ctl;
     a.parity = parity;
     a.dt_in = dt_in;
-    auto launch = stage_launcher(s->cfg.precision);
     // stage 1: U^n (A) -> U* (B)
     a.src = s->A;
     a.un = s->A;
     a.dst = s->B;
     a.dt_log = dt_log;
-    launch(1, s->shape, &s->mapA[s->shape], &s->mapE1[s->shape], a, s->stream);
+    launch_planned(s, 1, &s->mapA[stage_plan(s, 1)], a);
     a.dt_log = nullptr;
     launch_boundary(s->g, s->B, s->row2, nullptr, 0, s->stream);
     // stage 2: (U*, U^n) -> U^{n+1} in A
     a.src = s->B;
     a.un = s->A;
     a.dst = s->A;
-    launch(2, s->shape2, &s->mapB[s->shape2], &s->mapE2[s->shape2], a, s->stream);
+    launch_planned(s, 2, &s->mapB[stage_plan(s, 2)], a);
     launch_boundary_mirrored(s->g, s->A, s->row2, s->ctl, parity ^ 1, mirror, s->stream);
 }
 
@@ -525,10 +564,11 @@ int rmhd2d_create(const rmhd2d_config *cfg, rmhd2d_solver **out)
         cudaMemsetAsync(s->ctl, 0, sizeof(Control), s->stream) != cudaSuccess ||
         cudaStreamSynchronize(s->stream) != cudaSuccess)
         return bail(RMHD2D_ERR_CUDA, "device memset failed");
-    for (int sh = 0; sh < NSHAPE; ++sh)
+    for (int sh = 0; sh < NSHAPE_ALL; ++sh)
         if (!encode_state_map(&s->mapA[sh], g, s->A, stage_ui(1, sh), shape_uj(sh)) ||
             !encode_state_map(&s->mapB[sh], g, s->B, stage_ui(2, sh), shape_uj(sh)))
             return bail(RMHD2D_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    default_shapes(s);
     *out = s;
     return RMHD2D_OK;
 }
@@ -608,7 +648,7 @@ int rmhd2d_set_eta_table(rmhd2d_solver *s, const double *host_eta)
         CK(cudaMalloc(&s->eta, (size_t)s->g.plane * sizeof(double)));
         CK(cudaMemsetAsync(s->eta, 0, (size_t)s->g.plane * sizeof(double), s->stream));
         bool ok = true;
-        for (int sh = 0; sh < NSHAPE; ++sh)
+        for (int sh = 0; sh < NSHAPE_ALL; ++sh)
             ok = ok && encode_eta_map(&s->mapE1[sh], s->g, s->eta, stage_ui(1, sh), shape_uj(sh)) &&
                  encode_eta_map(&s->mapE2[sh], s->g, s->eta, stage_ui(2, sh), shape_uj(sh));
         if (!ok) {
@@ -772,15 +812,14 @@ int rmhd2d_profile_step(rmhd2d_solver *s, float *ms4)
     a.row2 = s->g.bc_x == BC_SYMMETRIC ? s->row2 : nullptr;
     a.ctl = s->ctl;
     a.parity = parity;
-    auto launch = stage_launcher(s->cfg.precision);
     CK(cudaEventRecord(ev[0], s->stream));
     a.src = s->A; a.un = s->A; a.dst = s->B;
-    launch(1, s->shape, &s->mapA[s->shape], &s->mapE1[s->shape], a, s->stream);
+    launch_planned(s, 1, &s->mapA[stage_plan(s, 1)], a);
     CK(cudaEventRecord(ev[1], s->stream));
     launch_boundary(s->g, s->B, s->row2, nullptr, 0, s->stream);
     CK(cudaEventRecord(ev[2], s->stream));
     a.src = s->B; a.un = s->A; a.dst = s->A;
-    launch(2, s->shape2, &s->mapB[s->shape2], &s->mapE2[s->shape2], a, s->stream);
+    launch_planned(s, 2, &s->mapB[stage_plan(s, 2)], a);
     CK(cudaEventRecord(ev[3], s->stream));
     launch_boundary(s->g, s->A, s->row2, s->ctl, parity ^ 1, s->stream);
     CK(cudaEventRecord(ev[4], s->stream));
@@ -881,6 +920,7 @@ int rmhd2d_set_stage_shapes(rmhd2d_solver *s, int shape1, int shape2)
     destroy_graphs(s);
     s->shape = shape1;
     s->shape2 = shape2;
+    s->own[0] = s->own[1] = -1;
     return RMHD2D_OK;
 }
 
@@ -972,9 +1012,14 @@ int rmhd2d_autotune(rmhd2d_solver *s, int trial_steps, int *best_shape)
     // Each stage's launch is timed by itself (the two stages read and write
     // different tiles and buffers), so the fastest shape is picked per stage:
     // the median over trial steps of each stage's CUDA-event time.
+    // On a small grid its own shape is tried too, and taken where it beats
+    // every public one.
     s->tuning_ms.assign(2 * NSHAPE, 0.f);
-    for (int sh = 0; sh < NSHAPE && rc == RMHD2D_OK; ++sh) {
-        rc = rmhd2d_set_stage_shapes(s, sh, sh);
+    const bool small = small_grid(s->g);
+    float small_ms[2] = {0.f, 0.f};
+    for (int sh = 0; sh < (small ? NSHAPE_ALL : NSHAPE) && rc == RMHD2D_OK; ++sh) {
+        rc = rmhd2d_set_stage_shapes(s, sh < NSHAPE ? sh : 0, sh < NSHAPE ? sh : 0);
+        if (sh == SHAPE_SMALL) s->own[0] = s->own[1] = SHAPE_SMALL;
         if (!rc) rc = rmhd2d_run(s, 2);                          // warm-up
         std::vector<float> t1, t2;
         for (int k = 0; k < trial_steps && !rc; ++k) {
@@ -986,8 +1031,9 @@ int rmhd2d_autotune(rmhd2d_solver *s, int trial_steps, int *best_shape)
         if (!rc) {
             std::sort(t1.begin(), t1.end());
             std::sort(t2.begin(), t2.end());
-            s->tuning_ms[2 * sh] = t1[t1.size() / 2];
-            s->tuning_ms[2 * sh + 1] = t2[t2.size() / 2];
+            float *to = sh == SHAPE_SMALL ? small_ms : &s->tuning_ms[2 * sh];
+            to[0] = t1[t1.size() / 2];
+            to[1] = t2[t2.size() / 2];
         }
     }
     const int rc2 = snapshot_restore(s, sn);
@@ -999,6 +1045,8 @@ int rmhd2d_autotune(rmhd2d_solver *s, int trial_steps, int *best_shape)
         if (s->tuning_ms[2 * sh + 1] < s->tuning_ms[2 * b2 + 1]) b2 = sh;
     }
     rc = rmhd2d_set_stage_shapes(s, b1, b2);
+    if (small && small_ms[0] < s->tuning_ms[2 * b1]) s->own[0] = SHAPE_SMALL;
+    if (small && small_ms[1] < s->tuning_ms[2 * b2 + 1]) s->own[1] = SHAPE_SMALL;
     if (best_shape) *best_shape = b1;
     return rc;
 }
@@ -1508,17 +1556,16 @@ int rmhd2d_slab_stage(rmhd2d_solver *s, int stage)
     a.row2 = s->g.bc_x == BC_SYMMETRIC ? s->row2 : nullptr;
     a.ctl = s->ctl;
     a.parity = s->parity;
-    auto launch = stage_launcher(s->cfg.precision);
     if (stage == 1) {
         a.src = s->A;
         a.un = s->A;
         a.dst = s->B;
-        launch(1, s->shape, &s->mapA[s->shape], &s->mapE1[s->shape], a, s->stream);
+        launch_planned(s, 1, &s->mapA[stage_plan(s, 1)], a);
     } else {
         a.src = s->B;
         a.un = s->A;
         a.dst = s->A;
-        launch(2, s->shape2, &s->mapB[s->shape2], &s->mapE2[s->shape2], a, s->stream);
+        launch_planned(s, 2, &s->mapB[stage_plan(s, 2)], a);
     }
     CK(cudaGetLastError());
     return RMHD2D_OK;
@@ -1686,11 +1733,12 @@ extern "C" int rmhd2d_adjoint_forward(rmhd2d_solver *s, int nsteps, int checkpoi
     if (tape) {
         // every step reads U^n from and writes U* and U^{n+1} into the
         // segment slots, through each slot's own tensor maps
+        const int k1 = stage_plan(s, 1), k2 = stage_plan(s, 2);
         w->map0.resize(nsteps);
         w->map1.resize(nsteps);
         for (int k = 0; k < nsteps; ++k)
-            if (!encode_state_map(&w->map0[k], g, w->seg0 + (size_t)k * sd, stage_ui(1, s->shape), shape_uj(s->shape)) ||
-                !encode_state_map(&w->map1[k], g, w->seg1 + (size_t)k * sd, stage_ui(2, s->shape2), shape_uj(s->shape2)))
+            if (!encode_state_map(&w->map0[k], g, w->seg0 + (size_t)k * sd, stage_ui(1, k1), shape_uj(k1)) ||
+                !encode_state_map(&w->map1[k], g, w->seg1 + (size_t)k * sd, stage_ui(2, k2), shape_uj(k2)))
                 return fail(s, RMHD2D_ERR_CUDA, "cuTensorMapEncodeTiled failed for the adjoint's trajectory slots");
         CK(cudaMemcpyAsync(w->seg0, s->A, sd * sizeof(double), cudaMemcpyDeviceToDevice, s->stream));
         for (int n = 0; n < nsteps; ++n) {
@@ -1749,11 +1797,12 @@ extern "C" int rmhd2d_adjoint_backward(rmhd2d_solver *s, const double *host_seed
     // tensor maps of the segment slots for the solver's tile shape (a kept
     // trajectory is read as it is: nothing is recomputed)
     if (!w->tape) {
+        const int k1 = stage_plan(s, 1), k2 = stage_plan(s, 2);
         w->map0.resize(w->interval);
         w->map1.resize(w->interval);
         for (int k = 0; k < w->interval; ++k)
-            if (!encode_state_map(&w->map0[k], g, w->seg0 + (size_t)k * sd, stage_ui(1, s->shape), shape_uj(s->shape)) ||
-                !encode_state_map(&w->map1[k], g, w->seg1 + (size_t)k * sd, stage_ui(2, s->shape2), shape_uj(s->shape2)))
+            if (!encode_state_map(&w->map0[k], g, w->seg0 + (size_t)k * sd, stage_ui(1, k1), shape_uj(k1)) ||
+                !encode_state_map(&w->map1[k], g, w->seg1 + (size_t)k * sd, stage_ui(2, k2), shape_uj(k2)))
                 return fail(s, RMHD2D_ERR_CUDA, "cuTensorMapEncodeTiled failed for the adjoint's segment states");
     }
     int rc = set_fixed_dt_mode(s, 1);

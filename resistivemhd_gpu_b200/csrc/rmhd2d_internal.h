@@ -65,20 +65,33 @@ enum KernelError { KERR_NONE = 0, KERR_TMA_TIMEOUT = 1 };
 // Which is fastest for a variant and grid is the autotuners' question.
 constexpr int HALO = 3;
 constexpr int NSHAPE = 6;
-constexpr int shape_tj(int shape) { return shape == 1 ? 16 : shape == 3 ? 64 : 32; }
+// SHAPE_SMALL, after them, is no public shape index: 4 x 16 cells (192 and 148
+// interfaces) for 192 threads, one interface each, for grids too small to
+// fill the SMs, where a stage takes as long as one block.
+constexpr int SHAPE_SMALL = NSHAPE;
+constexpr int NSHAPE_ALL = NSHAPE + 1;
+constexpr int SM_COUNT = 148;
+constexpr int shape_tj(int shape) { return shape == 1 || shape == SHAPE_SMALL ? 16 : shape == 3 ? 64 : 32; }
 constexpr int stage_ti(int stage, int shape)
 {
-    return shape == 0 ? (stage == 1 ? 8 : 9)
+    return shape == SHAPE_SMALL ? 4
+         : shape == 0 ? (stage == 1 ? 8 : 9)
          : shape == 5 ? (stage == 1 ? 6 : 7)
          : shape >= 3 ? 8 : (stage == 1 ? 16 : 18);
 }
 constexpr int stage_ui(int stage, int shape) { return stage_ti(stage, shape) + 2 * HALO; }
 constexpr int shape_uj(int shape) { return shape_tj(shape) + 2 * HALO; }  // TMA inner box: UJ * 8 B, a multiple of 16
-constexpr int shape_threads(int shape) { return shape == 2 ? 640 : shape == 3 ? 512 : shape >= 4 ? 256 : 320; }
-constexpr int shape_max_ctas(int shape) { return shape == 2 || shape == 3 ? 1 : shape >= 4 ? 3 : 2; }   // CTAs per SM that fit
+constexpr int shape_threads(int shape)
+{
+    return shape == SHAPE_SMALL ? 192 : shape == 2 ? 640 : shape == 3 ? 512 : shape >= 4 ? 256 : 320;
+}
+constexpr int shape_max_ctas(int shape)   // CTAs per SM that fit
+{
+    return shape == SHAPE_SMALL ? 2 : shape == 2 || shape == 3 ? 1 : shape >= 4 ? 3 : 2;
+}
 constexpr bool shapes_have_a_thread_per_cell()
 {
-    for (int s = 0; s < NSHAPE; ++s)
+    for (int s = 0; s < NSHAPE_ALL; ++s)
         if (shape_threads(s) < stage_ti(2, s) * shape_tj(s) || shape_threads(s) < stage_ti(1, s) * shape_tj(s))
             return false;
     return true;

@@ -777,6 +777,7 @@ template <class F> static void with_stage_shape(int stage, int shape, const F &f
     RMHD_SHAPE_CASE(2)
     RMHD_SHAPE_CASE(3)
     RMHD_SHAPE_CASE(4)
+    RMHD_SHAPE_CASE(SHAPE_SMALL)
     default: RMHD_SHAPE_CASE(5)
     }
 #undef RMHD_SHAPE_CASE
@@ -852,13 +853,15 @@ struct LaunchBatch {
     cudaStream_t stream;
     template <int ST, int SH> void operator()() const
     {
-        using T = Tile<ST, SH>;
-        set_smem_attributes(stage_batch_kernel<ST, SH>, T::SMEM_BYTES, T::CTAS);
-        const BatchRun *r = runs;
-        const CUtensorMap *m = maps;
-        const TileRef *t = tiles;
-        const int n = ntiles, c = ctas, par = parity;
-        stage_batch_kernel<ST, SH><<<c, T::THREADS, T::SMEM_BYTES, stream>>>(r, m, t, n, par);
+        if constexpr (SH < NSHAPE) {   // batches run the public shapes
+            using T = Tile<ST, SH>;
+            set_smem_attributes(stage_batch_kernel<ST, SH>, T::SMEM_BYTES, T::CTAS);
+            const BatchRun *r = runs;
+            const CUtensorMap *m = maps;
+            const TileRef *t = tiles;
+            const int n = ntiles, c = ctas, par = parity;
+            stage_batch_kernel<ST, SH><<<c, T::THREADS, T::SMEM_BYTES, stream>>>(r, m, t, n, par);
+        }
     }
 };
 
