@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "aux_kernels.h"
+#include "cell_block.cuh"
 #include "physics.cuh"
 
 namespace rmhd2d {
@@ -375,23 +376,32 @@ __global__ void snapshot_row2_kernel(Grid g, const double *s, double *row2)
 }
 
 // CFL rate over every cell (resistiveMHD_2D.cu:247-291) and the NaN-energy
-// test (resistiveMHD_2D.cu:294-309).
-__global__ void rate_kernel(Grid g, const double *s, Control *ctl, int slot, int set_crash)
+// test (resistiveMHD_2D.cu:294-309).  Each block walks several 8 x 32 groups
+// of cells and adds one atomic to the reduction.
+constexpr int RATE_ROWS = 8;
+__global__ void __launch_bounds__(32 * RATE_ROWS) rate_kernel(Grid g, const double *s, Control *ctl, int slot,
+                                                              int set_crash)
 {
-    const long long n = (long long)g.nx * g.ny;
+    __shared__ unsigned long long wmax[RATE_ROWS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned across = (unsigned)(g.ny + 31) / 32u, groups = CellBlock<RATE_ROWS>::blocks(g);
+    const long long P = g.plane;
+    MdDiv dd;
+    const double ydx = dd.recip(g.dx), ydy = dd.recip(g.dy);
     unsigned long long bits = 0ull;
     int nan_e = 0;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
-        if (halo_col(g, i)) continue;   // a slab's halo cells are reduced by their owner
+    for (unsigned b = blockIdx.x; b < groups; b += gridDim.x) {
+        const unsigned bi = b / across;
+        const int i = (int)(bi * RATE_ROWS) + warp, j = (int)((b - bi * across) * 32u) + lane;
+        // (a slab's halo cells are reduced by their owner)
+        if (i >= g.nx || j >= g.ny || halo_col(g, i)) continue;
         const long long k = at(g, i, j);
-        const long long P = g.plane;
         const double e = s[EN * P + k];
-        const double r = cfl_rate(s[RHO * P + k], s[MX * P + k], s[MY * P + k], s[MZ * P + k],
-                                  s[BXF * P + k], s[BYF * P + k], s[BZF * P + k], e, g.gamma, g.dx, g.dy);
-        const unsigned long long b = rate_bits(r);
-        bits = b > bits ? b : bits;
-        if (t == 0 && r != r) ctl->first_nan[slot] = 1;
+        const double r = cfl_rate_md(s[RHO * P + k], s[MX * P + k], s[MY * P + k], s[MZ * P + k], s[BXF * P + k],
+                                     s[BYF * P + k], s[BZF * P + k], e, g.gamma, g.dx, g.dy, ydx, ydy, dd.ok);
+        const unsigned long long o = rate_bits(r);
+        bits = o > bits ? o : bits;
+        if (i == 0 && j == 0 && r != r) ctl->first_nan[slot] = 1;
         nan_e |= (e != e);
     }
 #pragma unroll
@@ -399,8 +409,10 @@ __global__ void rate_kernel(Grid g, const double *s, Control *ctl, int slot, int
         const unsigned long long o = __shfl_xor_sync(0xffffffffu, bits, off);
         bits = o > bits ? o : bits;
     }
-    const int any_nan = __any_sync(0xffffffffu, nan_e);
-    if ((threadIdx.x & 31) == 0) {
+    if (lane == 0) wmax[warp] = bits;
+    const int any_nan = __syncthreads_or(nan_e);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < RATE_ROWS; ++w) bits = wmax[w] > bits ? wmax[w] : bits;
         atomicMax(&ctl->amax[slot], bits);
         if (set_crash && any_nan) atomicExch(&ctl->crashed, 1);
     }
@@ -543,7 +555,8 @@ void launch_snapshot_row2(const Grid &g, const double *s, double *row2, cudaStre
 
 void launch_rate(const Grid &g, const double *s, Control *ctl, int slot, int set_crash, cudaStream_t st)
 {
-    rate_kernel<<<grid_for((long long)g.nx * g.ny, 256), 256, 0, st>>>(g, s, ctl, slot, set_crash);
+    const unsigned groups = CellBlock<RATE_ROWS>::blocks(g), most = 148u * 8u;   // all resident at once
+    rate_kernel<<<groups < most ? groups : most, CellBlock<RATE_ROWS>::THREADS, 0, st>>>(g, s, ctl, slot, set_crash);
 }
 
 void launch_slab_halo(const Grid &g, double *s, double *buf, int col0, int to_buf, cudaStream_t st)

@@ -24,8 +24,8 @@
 // only ghost cells, which the boundary passes overwrite.
 #include <cuda_runtime.h>
 
-#include "adjoint_core.cuh"
 #include "aux_kernels.h"
+#include "cell_block.cuh"
 #include "contact.h"
 #include "physics.cuh"
 #include "rmhd2d_internal.h"
@@ -60,21 +60,6 @@ __device__ __forceinline__ double by_s(const Grid &g, const double *U, int i, in
     return j < g.ny - 1 ? 0.5 * (by_c(g, U, i, j) + by_c(g, U, i, j + 1)) : by_c(g, U, i, j);
 }
 
-// A cell of the cell-centred state in sweep order (hlld.cu:134-160 shuffles
-// the y sweep's cell to rho, rhoV, rhoW, rhoU, bY, bZ, bX, e).
-template <int DIR>
-__device__ __forceinline__ void sweep_cell(const Grid &g, const double *U, int i, int j, double *c)
-{
-    const long long k = at(g, i, j), P = g.plane;
-    if (DIR == 0) {
-        c[0] = U[RHO * P + k]; c[1] = U[MX * P + k]; c[2] = U[MY * P + k]; c[3] = U[MZ * P + k];
-        c[4] = bx_c(g, U, i, j); c[5] = by_c(g, U, i, j); c[6] = U[BZF * P + k]; c[7] = U[EN * P + k];
-    } else {
-        c[0] = U[RHO * P + k]; c[1] = U[MY * P + k]; c[2] = U[MZ * P + k]; c[3] = U[MX * P + k];
-        c[4] = by_c(g, U, i, j); c[5] = U[BZF * P + k]; c[6] = bx_c(g, U, i, j); c[7] = U[EN * P + k];
-    }
-}
-
 // F and G of every interface: HLLD::calculateFluxF / G (hlld.cu:110-233)
 // of the cell-centred state plus the resistive hook
 // (main_plasmoid.cu:175-290).  The x sweep is defined for 1 <= i <= nx-4,
@@ -87,15 +72,23 @@ __device__ __forceinline__ void sweep_cell(const Grid &g, const double *U, int i
 // of its CT_TI x CT_TJ cells from there, in the reference's order of
 // operations.  Divisions go through shared correctly rounded reciprocals
 // (MdDiv, with IEEE division where its guard fails), which give the
-// reference's quotients bit for bit.
-constexpr int CT_TI = 16, CT_TJ = 32, CT_THREADS = 256;
+// reference's quotients bit for bit.  The flux takes its common path in the
+// loop and the declined interfaces after it, as the stage kernels do: it then
+// fits 80 registers and three CTAs per SM (24 warps; FP64-issue bound).  Harris
+// 2048 x 1024: 382 us a launch at two CTAs with every candidate kept, 316 now;
+// at two CTAs the step took 1235 us, at three 1176.
+constexpr int CT_TI = 16, CT_TJ = 32, CT_THREADS = 256, CT_CTAS = 3;
 constexpr int CT_SI = CT_TI + 3, CT_SJ = CT_TJ + 3, CT_SC = CT_SI * CT_SJ;
 constexpr int CT_JI = CT_TI + 1, CT_JJ = CT_TJ + 1, CT_JC = CT_JI * CT_JJ;
 enum { S_RHO = 0, S_U, S_V, S_W, S_BXC, S_BYC, S_BZ, S_PX, S_PY, S_NF };
 enum { J_X = 0, J_Y, J_Z, J_NF };   // eta*Jx, eta*Jy, eta*Jz
 constexpr size_t CT_SMEM = (size_t)(S_NF * CT_SC + J_NF * CT_JC) * sizeof(double);
 
-__global__ void __launch_bounds__(CT_THREADS, 2) contact_flux_tiled_kernel(Grid g, const double *U, const double *eta,
+template <bool B> struct FullFlux {
+    static constexpr bool value = B;
+};
+
+__global__ void __launch_bounds__(CT_THREADS, CT_CTAS) contact_flux_tiled_kernel(Grid g, const double *U, const double *eta,
                                                                          double *F, double *G)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -166,80 +159,95 @@ __global__ void __launch_bounds__(CT_THREADS, 2) contact_flux_tiled_kernel(Grid 
     }
     __syncthreads();
 
-    for (int t = threadIdx.x; t < 2 * CT_TI * CT_TJ; t += CT_THREADS) {
+    MdDiv cg;
+    const double ygm1 = cg.recip(gm1);
+    const bool gm1_ok = cg.ok;
+    // One interface; false, with nothing stored, where the flux's common path
+    // declines it (hlld_flux_sel).  Full: the reference's arithmetic in full.
+    auto flux_at = [&](const int t, const auto full) -> bool {
         const int dir = t >= CT_TI * CT_TJ;
         const int r = t - dir * CT_TI * CT_TJ;
         const int li = r / CT_TJ, lj = r - li * CT_TJ;
         const int i = i0 + li, j = j0 + lj;
-        if (i >= g.nx || j >= g.ny) continue;
-        const int si = li + 1, sj = lj + 1;
-        double out[8];
+        if (i >= g.nx || j >= g.ny) return true;
+        double *o = (dir == 0 ? F : G) + at(g, i, j);
         const bool ok = dir == 0 ? (i >= 1 && i <= g.nx - 4) : (j >= 1 && j <= g.ny - 3);
         if (!ok) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) out[c] = qnan();
-        } else {
-            // sweep-order primitives of the four cells along the sweep
-            double q[4][8];
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int c = dir == 0 ? at_s(si - 1 + m, sj) : at_s(si, sj - 1 + m);
-                if (dir == 0) {
-                    q[m][0] = S[S_RHO][c]; q[m][1] = S[S_U][c]; q[m][2] = S[S_V][c]; q[m][3] = S[S_W][c];
-                    q[m][5] = S[S_BYC][c]; q[m][6] = S[S_BZ][c]; q[m][7] = S[S_PX][c];
-                } else {
-                    q[m][0] = S[S_RHO][c]; q[m][1] = S[S_V][c]; q[m][2] = S[S_W][c]; q[m][3] = S[S_U][c];
-                    q[m][5] = S[S_BZ][c]; q[m][6] = S[S_BXC][c]; q[m][7] = S[S_PY][c];
-                }
-                q[m][4] = 0.0;
-            }
-            // basic_param's interface-normal B of the left cell and its neighbour
-            {
-                const int nb = dir == 0 ? S_BXC : S_BYC;
-                const int c1 = at_s(si, sj), c2 = dir == 0 ? at_s(si + 1, sj) : at_s(si, sj + 1);
-                q[1][4] = XMUL(0.5, XADD(S[nb][c1], S[nb][c2]));
-            }
-            double L[8], R[8], f[8];
-            adj::muscl_states(q[0], q[1], q[2], q[3], g.eps, L, R);
-            const Prim PL{L[0], L[1], L[2], L[3], L[4], L[5], L[6], L[7]};
-            const Prim PR{R[0], R[1], R[2], R[3], R[4], R[5], R[6], R[7]};
-            hlld_flux<true>(PL, PR, g.gamma, g.eps, f);
-            if (dir == 0) {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) out[c] = f[c];
-            } else {
-                out[0] = f[0]; out[1] = f[3]; out[2] = f[1]; out[3] = f[2];
-                out[4] = f[6]; out[5] = f[4]; out[6] = f[5]; out[7] = f[7];
-            }
-            // the resistive hook (the reference's 0 < i < nx-2, 0 < j < ny-2)
-            if (i >= 1 && i <= g.nx - 3 && j >= 1 && j <= g.ny - 3) {
-                const int c0 = li * CT_JJ + lj;                         // eta*J of cell (i, j)
-                if (dir == 0) {
-                    const int c1 = c0 + CT_JJ;                          // (i + 1, j)
-                    const double etaJY = J[J_Y][c0], etaJZ = J[J_Z][c0];
-                    const double etaJYBZ = etaJY * bz(si, sj), etaJZBY = etaJZ * byc(si, sj);
-                    const double etaJYPlus1 = J[J_Y][c1], etaJZPlus1 = J[J_Z][c1];
-                    const double etaJYBZPlus1 = etaJYPlus1 * bz(si + 1, sj), etaJZBYPlus1 = etaJZPlus1 * byc(si + 1, sj);
-                    out[5] -= 0.5 * (etaJZ + etaJZPlus1);
-                    out[6] += 0.5 * (etaJY + etaJYPlus1);
-                    out[7] += 0.5 * (etaJYBZ + etaJYBZPlus1) - 0.5 * (etaJZBY + etaJZBYPlus1);
-                } else {
-                    const int c1 = c0 + 1;                              // (i, j + 1)
-                    const double etaJX = J[J_X][c0], etaJZ = J[J_Z][c0];
-                    const double etaJXBZ = etaJX * bz(si, sj), etaJZBX = etaJZ * bxc(si, sj);
-                    const double etaJXPlus1 = J[J_X][c1], etaJZPlus1 = J[J_Z][c1];
-                    const double etaJXBZPlus1 = etaJXPlus1 * bz(si, sj + 1), etaJZBXPlus1 = etaJZPlus1 * bxc(si, sj + 1);
-                    out[4] += 0.5 * (etaJZ + etaJZPlus1);
-                    out[6] -= 0.5 * (etaJX + etaJXPlus1);
-                    out[7] += 0.5 * (etaJZBX + etaJZBXPlus1) - 0.5 * (etaJXBZ + etaJXBZPlus1);
-                }
-            }
+            for (int c = 0; c < 8; ++c)
+                if (c != (dir == 0 ? BXF : BYF)) o[c * P] = qnan();
+            return true;
         }
-        double *o = (dir == 0 ? F : G) + at(g, i, j);
+        const int si = li + 1, sj = lj + 1;
+        // sweep-order primitives of the four cells along the sweep, MUSCL
+        // (muscl.cu:6-126)
+        const int c1 = at_s(si, sj), st = dir == 0 ? CT_SJ : 1;
+        const int order[7] = {S_RHO, dir == 0 ? S_U : S_V, dir == 0 ? S_V : S_W, dir == 0 ? S_W : S_U,
+                              dir == 0 ? S_BYC : S_BZ, dir == 0 ? S_BZ : S_BXC, dir == 0 ? S_PX : S_PY};
+        double qL[7], qR[7];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) o[c * P] = out[c];
+        for (int n = 0; n < 7; ++n) {
+            const double *q = S[order[n]] + c1;
+            const double qm = q[-st], q0 = q[0], qp = q[st], qpp = q[2 * st];
+            qL[n] = q0 + 0.5 * minmod(q0 - qm, qp - q0, g.eps);
+            qR[n] = qp - 0.5 * minmod(qp - q0, qpp - qp, g.eps);
+        }
+        // basic_param's interface-normal B of the left cell and its neighbour
+        const double *nb = S[dir == 0 ? S_BXC : S_BYC] + c1;
+        const double bn = 0.5 * (nb[0] + nb[st]);
+        const Prim L{qL[0], qL[1], qL[2], qL[3], bn, qL[4], qL[5], qL[6]};
+        const Prim R{qR[0], qR[1], qR[2], qR[3], bn, qR[4], qR[5], qR[6]};
+        double f[8];
+        if (full.value)
+            hlld_flux_ieee(L, R, g.gamma, g.eps, f);
+        else if (!hlld_flux_sel(L, R, g.gamma, g.eps, ygm1, gm1_ok, f))
+            return false;
+        // the resistive hook (the reference's 0 < i < nx-2, 0 < j < ny-2), and
+        // for the y sweep the un-permuted components (hlld.cu:170-194)
+        const bool hook = i >= 1 && i <= g.nx - 3 && j >= 1 && j <= g.ny - 3;
+        const int cj0 = li * CT_JJ + lj;                        // eta*J of cell (i, j)
+        if (dir == 0) {
+            double by = f[5], bzf = f[6], en = f[7];
+            if (hook) {
+                const int cj1 = cj0 + CT_JJ;                    // (i + 1, j)
+                const double etaJY = J[J_Y][cj0], etaJZ = J[J_Z][cj0];
+                const double etaJYBZ = etaJY * bz(si, sj), etaJZBY = etaJZ * byc(si, sj);
+                const double etaJYPlus1 = J[J_Y][cj1], etaJZPlus1 = J[J_Z][cj1];
+                const double etaJYBZPlus1 = etaJYPlus1 * bz(si + 1, sj), etaJZBYPlus1 = etaJZPlus1 * byc(si + 1, sj);
+                by -= 0.5 * (etaJZ + etaJZPlus1);
+                bzf += 0.5 * (etaJY + etaJYPlus1);
+                en += 0.5 * (etaJYBZ + etaJYBZPlus1) - 0.5 * (etaJZBY + etaJZBYPlus1);
+            }
+            o[RHO * P] = f[0]; o[MX * P] = f[1]; o[MY * P] = f[2]; o[MZ * P] = f[3];
+            o[BYF * P] = by; o[BZF * P] = bzf; o[EN * P] = en;
+        } else {
+            double bx = f[6], bzf = f[5], en = f[7];
+            if (hook) {
+                const int cj1 = cj0 + 1;                        // (i, j + 1)
+                const double etaJX = J[J_X][cj0], etaJZ = J[J_Z][cj0];
+                const double etaJXBZ = etaJX * bz(si, sj), etaJZBX = etaJZ * bxc(si, sj);
+                const double etaJXPlus1 = J[J_X][cj1], etaJZPlus1 = J[J_Z][cj1];
+                const double etaJXBZPlus1 = etaJXPlus1 * bz(si, sj + 1), etaJZBXPlus1 = etaJZPlus1 * bxc(si, sj + 1);
+                bx += 0.5 * (etaJZ + etaJZPlus1);
+                bzf -= 0.5 * (etaJX + etaJXPlus1);
+                en += 0.5 * (etaJZBX + etaJZBXPlus1) - 0.5 * (etaJXBZ + etaJXBZPlus1);
+            }
+            o[RHO * P] = f[0]; o[MX * P] = f[3]; o[MY * P] = f[1]; o[MZ * P] = f[2];
+            o[BXF * P] = bx; o[BZF * P] = bzf; o[EN * P] = en;
+        }
+        return true;
+    };
+    // the rare path after the loop, as in the stage kernels
+    unsigned redo = 0u;
+    for (int t = threadIdx.x, p = 0; t < 2 * CT_TI * CT_TJ; t += CT_THREADS, ++p)
+        redo |= flux_at(t, FullFlux<false>{}) ? 0u : 1u << p;
+    if (redo) {
+        for (int t = threadIdx.x, p = 0; t < 2 * CT_TI * CT_TJ; t += CT_THREADS, ++p)
+            if ((redo >> p) & 1u) flux_at(t, FullFlux<true>{});
     }
 }
+
+using Cells = CellBlock<8>;   // of the per-cell kernels below
 
 __global__ void contact_begin_kernel(Grid g, Control *ctl, int parity)
 {
@@ -258,16 +266,10 @@ __global__ void contact_begin_kernel(Grid g, Control *ctl, int parity)
 // 0 < i < nx-1, 0 < j < ny-1, from U's face B, smoothed (stage 1) or as
 // stored (stage 2).
 template <bool SMOOTHED>
-__global__ void contact_ref_kernel(Grid g, const double *U, const double *eta, double *ref)
+__device__ __forceinline__ double reference_emf(const Grid &g, const double *U, const double *eta, int i, int j)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.nx * g.ny) return;
-    const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
     const long long k = at(g, i, j), P = g.plane;
-    if (!(i > 0 && i < g.nx - 1 && j > 0 && j < g.ny - 1)) {
-        ref[k] = qnan();
-        return;
-    }
+    if (!(i > 0 && i < g.nx - 1 && j > 0 && j < g.ny - 1)) return qnan();
     auto BX = [&](int ii, int jj) { return SMOOTHED ? bx_s(g, U, ii, jj) : U[BXF * P + at(g, ii, jj)]; };
     auto BY = [&](int ii, int jj) { return SMOOTHED ? by_s(g, U, ii, jj) : U[BYF * P + at(g, ii, jj)]; };
     const double dx = g.dx, dy = g.dy;
@@ -297,19 +299,29 @@ __global__ void contact_ref_kernel(Grid g, const double *U, const double *eta, d
         IeeeDiv id;
         r = ref_of(id);
     }
-    ref[k] = r;
+    return r;
+}
+
+// The reference EMF of every cell of the stage-2 result (the stage-1 one's is
+// formed by its update, which reads the same cells).
+__global__ void contact_ref_kernel(Grid g, const double *U, const double *eta, double *ref)
+{
+    int i, j;
+    if (!Cells::cell(g, i, j)) return;
+    ref[at(g, i, j)] = reference_emf<false>(g, U, eta, i, j);
 }
 
 // The stage updates (resistiveMHD_2D.cu:53-130 functors, over k >= ny), all
-// 8 fields, face B as shift + back-to-face leave it.
+// 8 fields, face B as shift + back-to-face leave it.  Stage 1 also forms the
+// reference EMF of U^n, from the same reads.
 template <int STAGE>
 __global__ void contact_update_kernel(Grid g, const double *Un, const double *Ub, const double *F, const double *G,
-                                      const Control *ctl, double *dst)
+                                      const Control *ctl, double *dst, const double *eta, double *ref)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.nx * g.ny) return;
-    const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
+    int i, j;
+    if (!Cells::cell(g, i, j)) return;
     const long long k = at(g, i, j), P = g.plane;
+    if (STAGE == 1) ref[k] = reference_emf<true>(g, Un, eta, i, j);
     if (i == 0) {
         // outside the update range: stage 1 keeps U^n (copied before the
         // smoothing); stage 2 keeps U^n as the smoothing left it
@@ -329,9 +341,9 @@ __global__ void contact_update_kernel(Grid g, const double *Un, const double *Ub
     for (int c = 0; c < NFIELD; ++c) {
         // the flat k - 1 neighbour of j = 0 is the previous column's last
         // cell, whose G entry is NaN
-        const double gm = j >= 1 ? G[c * P + k - 1] : qnan();
-        const double div = rdx * (F[c * P + k] - F[c * P + km]);
-        const double dvg = rdy * (G[c * P + k] - gm);
+        // (F of bX and G of bY are identically 0 and not stored; u - 0 is u)
+        const double div = c == BXF ? 0.0 : rdx * (F[c * P + k] - F[c * P + km]);
+        const double dvg = c == BYF ? 0.0 : rdy * (G[c * P + k] - (j >= 1 ? G[c * P + k - 1] : qnan()));
         double u = Un[c * P + k];
         if (c == BXF) u = bx_s(g, Un, i, j);
         if (c == BYF) u = by_s(g, Un, i, j);
@@ -410,9 +422,8 @@ __device__ __forceinline__ double corner_ez(const Grid &g, const StageEmf &o, co
 // Every corner EMF once (corner_ez), NaN where it is undefined.
 __global__ void contact_corner_kernel(Grid g, StageEmf o, StageEmf n, double *E)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.nx * g.ny) return;
-    const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
+    int i, j;
+    if (!Cells::cell(g, i, j)) return;
     E[at(g, i, j)] = corner_ez(g, o, n, i, j);
 }
 
@@ -420,9 +431,8 @@ __global__ void contact_corner_kernel(Grid g, StageEmf o, StageEmf n, double *E)
 // state from the stage-2 result C; E holds the corner EMFs.
 __global__ void contact_ct_kernel(Grid g, const double *E, const double *C, const Control *ctl, double *A)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.nx * g.ny) return;
-    const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
+    int i, j;
+    if (!Cells::cell(g, i, j)) return;
     const long long k = at(g, i, j), P = g.plane;
 #pragma unroll
     for (int c = 0; c < NFIELD; ++c)
@@ -438,15 +448,12 @@ __global__ void contact_ct_kernel(Grid g, const double *E, const double *C, cons
     }
 }
 
-int blocks_for(long long n, int threads) { return (int)((n + threads - 1) / threads); }
-
 }  // namespace
 
 void enqueue_contact_step(const ContactStep &c, cudaStream_t st)
 {
     const Grid &g = c.g;
-    const long long n = (long long)g.nx * g.ny;
-    const int b256 = blocks_for(n, 256);
+    const unsigned cells = Cells::blocks(g);
     const dim3 flux_grid((g.ny + CT_TJ - 1) / CT_TJ, (g.nx + CT_TI - 1) / CT_TI);
     auto boundary = [&](double *state) {
         if (g.bc_x == BC_SYMMETRIC) launch_snapshot_row2(g, state, c.row2, st);
@@ -456,18 +463,17 @@ void enqueue_contact_step(const ContactStep &c, cudaStream_t st)
     contact_begin_kernel<<<1, 32, 0, st>>>(g, c.ctl, c.parity);
     // stage 1
     contact_flux_tiled_kernel<<<flux_grid, CT_THREADS, CT_SMEM, st>>>(g, c.A, c.eta, c.F1, c.G1);
-    contact_ref_kernel<true><<<b256, 256, 0, st>>>(g, c.A, c.eta, c.R1);
-    contact_update_kernel<1><<<b256, 256, 0, st>>>(g, c.A, nullptr, c.F1, c.G1, c.ctl, c.B);
+    contact_update_kernel<1><<<cells, Cells::THREADS, 0, st>>>(g, c.A, nullptr, c.F1, c.G1, c.ctl, c.B, c.eta, c.R1);
     boundary(c.B);
     // stage 2
     contact_flux_tiled_kernel<<<flux_grid, CT_THREADS, CT_SMEM, st>>>(g, c.B, c.eta, c.F2, c.G2);
-    contact_update_kernel<2><<<b256, 256, 0, st>>>(g, c.A, c.B, c.F2, c.G2, c.ctl, c.C);
+    contact_update_kernel<2><<<cells, Cells::THREADS, 0, st>>>(g, c.A, c.B, c.F2, c.G2, c.ctl, c.C, nullptr, nullptr);
     boundary(c.C);
-    contact_ref_kernel<false><<<b256, 256, 0, st>>>(g, c.C, c.eta, c.R2);
+    contact_ref_kernel<<<cells, Cells::THREADS, 0, st>>>(g, c.C, c.eta, c.R2);
     // CT with the two stages' mean contact EMF, then the boundary and the
     // next step's CFL rate and crash flag
-    contact_corner_kernel<<<b256, 256, 0, st>>>(g, StageEmf{c.F1, c.G1, c.R1}, StageEmf{c.F2, c.G2, c.R2}, c.E);
-    contact_ct_kernel<<<b256, 256, 0, st>>>(g, c.E, c.C, c.ctl, c.A);
+    contact_corner_kernel<<<cells, Cells::THREADS, 0, st>>>(g, StageEmf{c.F1, c.G1, c.R1}, StageEmf{c.F2, c.G2, c.R2}, c.E);
+    contact_ct_kernel<<<cells, Cells::THREADS, 0, st>>>(g, c.E, c.C, c.ctl, c.A);
     boundary(c.A);
     launch_rate(g, c.A, c.ctl, c.parity ^ 1, 1, st);
 }

@@ -154,7 +154,7 @@ __device__ __forceinline__ double rcp_nr(double a)
 __device__ __forceinline__ double rcp_rn_md(double b)
 {
     double y;
-#if defined(RMHD_HOST_EMULATION)
+#if !defined(__CUDA_ARCH__)
     // a seed with the precision of the hardware's (its low 28 significand
     // bits cleared), so that a host build exercises the refinement
     {
