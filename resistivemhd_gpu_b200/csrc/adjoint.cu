@@ -29,6 +29,7 @@
 #include "adjoint.h"
 #include "adjoint_common.cuh"
 #include "adjoint_core.cuh"
+#include "cell_block.cuh"
 
 namespace rmhd2d {
 
@@ -39,15 +40,16 @@ namespace {
 using namespace adjk;
 using adj::recon_comp;
 
-constexpr int ADJ_THREADS = 128;
+using IfaceCells = CellBlock<4>;
+using GatherCells = CellBlock<8>;
+using CenterCells = CellBlock<8>;
 
-__global__ void __launch_bounds__(ADJ_THREADS, 3) adj_iface_kernel(AdjStageArgs a)
+__global__ void __launch_bounds__(IfaceCells::THREADS, 3) adj_iface_kernel(AdjStageArgs a)
 {
     const Grid &g = a.g;
     const int dir = blockIdx.y;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.nx * g.ny) return;
-    const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
+    int i, j;
+    if (!IfaceCells::cell(g, i, j)) return;
     const long long k = at(g, i, j), P = g.plane;
     double *out = a.IF + (long long)dir * IF_PLANES * P + k;
     if (!iface_live(g, dir, i, j)) {
@@ -130,12 +132,11 @@ __device__ __forceinline__ void gather_sweep(const AdjStageArgs &a, int dir, int
     for (int s = 0; s < 8; ++s) nat_bar[sweep_field(dir, s)] += cb[s];
 }
 
-__global__ void __launch_bounds__(ADJ_THREADS, 6) adj_gather_kernel(AdjStageArgs a)
+__global__ void __launch_bounds__(GatherCells::THREADS, 3) adj_gather_kernel(AdjStageArgs a)
 {
     const Grid &g = a.g;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.nx * g.ny) return;
-    const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
+    int i, j;
+    if (!GatherCells::cell(g, i, j)) return;
     const long long k = at(g, i, j), P = g.plane;
     double wb[8];
 #pragma unroll
@@ -172,9 +173,8 @@ __global__ void __launch_bounds__(ADJ_THREADS, 6) adj_gather_kernel(AdjStageArgs
 __global__ void __launch_bounds__(256) adj_center_kernel(AdjStageArgs a)
 {
     const Grid &g = a.g;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.nx * g.ny) return;
-    const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
+    int i, j;
+    if (!CenterCells::cell(g, i, j)) return;
     const long long k = at(g, i, j), P = g.plane;
     const double *tx = a.tmp, *ty = a.tmp + P;
     const double cbx = (i >= 1 ? 0.5 : 1.0) * tx[k] + (i + 1 < g.nx ? 0.5 * tx[at(g, i + 1, j)] : 0.0);
@@ -251,13 +251,17 @@ __global__ void periodic_transpose_kernel(Grid g, double *Ub)
 //   bY(i,1) = bY(i,2) + (bX(i,2) - bX(i-1,2)) dy/dx      (bX(.,2) a copy of row 3)
 //   bY(i,0) = bY(i,1) + (bX(i,1) - bX(i-1,1)) dy/dx      (bX(.,1) a copy of row 4)
 // The transposes run in the opposite order, y then x, in gather form: a
-// thread owns one column (y) or one row (x), takes the chain adjoints of
-// its own and of the next column or row, and writes only its own entries;
-// the ghost entries it reads are zeroed by a separate launch after it.  The
-// x pass at row 3 reads the lower wall face bY(c,2) before the y pass
-// replaces it -- in the step, the stage-1 CT result (row2) -- so the x
-// transpose leaves that adjoint in the ghost entry (c,2) of the interior
-// columns, where the stage-1 reverse takes it as the CT'd face's.
+// thread owns one field of one column (y) or one row (x), takes the chain
+// adjoints of its own and of the next column or row, writes only its own
+// entries, and clears the ghost entries that only it reads.  Those that a
+// neighbour's chain reads too -- BYF in the y pass, BXF in the x pass -- are
+// cleared by the launch after it.  Every value is loaded before the first
+// store: with one thread per line and all fields' read-modify-writes in a
+// row, each waited for the one before it (150 x 90: 27 + 18 us per transpose,
+// now 3.5 + 3.5).  The x pass at row 3 reads the lower wall face bY(c,2)
+// before the y pass replaces it -- in the step, the stage-1 CT result (row2)
+// -- so the x transpose leaves that adjoint in the ghost entry (c,2) of the
+// interior columns, where the stage-1 reverse takes it as the CT'd face's.
 
 // Running sums of a lower and an upper chain's output adjoints: t1 = the
 // sum of all three, t2 = the outer two, t3 = the outermost.
@@ -270,116 +274,158 @@ __device__ __forceinline__ ChainAdj chain_adj(double inner, double middle, doubl
     return ChainAdj{inner + middle + outer, middle + outer, outer};
 }
 
+// The twelve entries of one field along a line of n cells that a wall's
+// transpose touches: ghosts 0..2 and n-3..n-1 (g), interior 3..5 and n-6..n-4
+// (v), `st` doubles apart from p on.
+struct WallLine {
+    double g[6], v[6];
+    __device__ __forceinline__ WallLine(const double *p, int n, long long st)
+    {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            g[q] = p[q * st];
+            v[q] = p[(3 + q) * st];
+            v[3 + q] = p[(n - 6 + q) * st];
+            g[3 + q] = p[(n - 3 + q) * st];
+        }
+    }
+    // Adds what the ghosts were copied from: periodic (ghost q <- n-6+q,
+    // n-3+q <- 3+q) or mirror (2 <- 3, 1 <- 4, 0 <- 5 and their twins).
+    __device__ __forceinline__ void add_copies(bool periodic)
+    {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            v[3 + q] += periodic ? g[q] : g[5 - q];
+            v[q] += periodic ? g[3 + q] : g[2 - q];
+        }
+    }
+    __device__ __forceinline__ void store(double *p, int n, long long st, bool clear_ghosts) const
+    {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            p[(3 + q) * st] = v[q];
+            p[(n - 6 + q) * st] = v[3 + q];
+            if (clear_ghosts) {
+                p[q * st] = 0.0;
+                p[(n - 3 + q) * st] = 0.0;
+            }
+        }
+    }
+};
+
+// One thread per column and field (blockIdx.y).
 template <int BY> __global__ void ytrans_kernel(Grid g, double *Ub)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, f = (int)blockIdx.y;
     if (i >= g.nx) return;
     const long long P = g.plane;
     const int ny = g.ny;
-    auto L = [&](int f, int ii, int jj) -> double & { return Ub[f * P + at(g, ii, jj)]; };
-    if (BY == BC_PERIODIC) {
-#pragma unroll
-        for (int f = 0; f < NFIELD; ++f)
-            for (int q = 0; q < 3; ++q) {
-                L(f, i, ny - 6 + q) += L(f, i, q);
-                L(f, i, 3 + q) += L(f, i, ny - 3 + q);
-            }
+    double *p = Ub + f * P + at(g, i, 0);
+    WallLine w(p, ny, 1);
+    if (BY == BC_PERIODIC || (f != BXF && f != BYF)) {
+        w.add_copies(BY == BC_PERIODIC);
+        w.store(p, ny, 1, true);
         return;
     }
-    const double c = g.dy / g.dx;
-    auto lower = [&](int col) { return chain_adj(L(BYF, col, 2), L(BYF, col, 1), L(BYF, col, 0)); };
-    auto upper = [&](int col) { return chain_adj(L(BYF, col, ny - 3), L(BYF, col, ny - 2), L(BYF, col, ny - 1)); };
+    auto B = [&](int col, int j) -> double { return Ub[BYF * P + at(g, col, j)]; };
+    auto lower = [&](int col) { return chain_adj(B(col, 2), B(col, 1), B(col, 0)); };
+    auto upper = [&](int col) { return chain_adj(B(col, ny - 3), B(col, ny - 2), B(col, ny - 1)); };
     const ChainAdj lo = lower(i), up = upper(i);
+    if (f == BYF) {
+        w.v[0] += lo.t1;
+        w.v[5] += up.t1;
+        w.store(p, ny, 1, false);
+        return;
+    }
     // chain terms on bX: this column's (i > 0) and the next column's
+    const double c = g.dy / g.dx;
     const ChainAdj z{0.0, 0.0, 0.0};
     const ChainAdj lo_own = i > 0 ? lo : z, up_own = i > 0 ? up : z;
     const ChainAdj lo_nxt = i + 1 < g.nx ? lower(i + 1) : z, up_nxt = i + 1 < g.nx ? upper(i + 1) : z;
-    L(BYF, i, 3) += lo.t1;
-    L(BYF, i, ny - 4) += up.t1;
-    L(BXF, i, 3) += L(BXF, i, 2) + c * (lo_own.t1 - lo_nxt.t1) + c * (lo_own.t2 - lo_nxt.t2);
-    L(BXF, i, 4) += L(BXF, i, 1) + c * (lo_own.t3 - lo_nxt.t3);
-    L(BXF, i, 5) += L(BXF, i, 0);
-    L(BXF, i, ny - 4) += L(BXF, i, ny - 3) - c * (up_own.t1 - up_nxt.t1);
-    L(BXF, i, ny - 5) += L(BXF, i, ny - 2) - c * (up_own.t2 - up_nxt.t2);
-    L(BXF, i, ny - 6) += L(BXF, i, ny - 1) - c * (up_own.t3 - up_nxt.t3);
-#pragma unroll
-    for (int f = 0; f < NFIELD; ++f) {
-        if (f == BXF || f == BYF) continue;
-        L(f, i, 3) += L(f, i, 2);
-        L(f, i, 4) += L(f, i, 1);
-        L(f, i, 5) += L(f, i, 0);
-        L(f, i, ny - 4) += L(f, i, ny - 3);
-        L(f, i, ny - 5) += L(f, i, ny - 2);
-        L(f, i, ny - 6) += L(f, i, ny - 1);
-    }
+    w.v[0] += w.g[2] + c * (lo_own.t1 - lo_nxt.t1) + c * (lo_own.t2 - lo_nxt.t2);
+    w.v[1] += w.g[1] + c * (lo_own.t3 - lo_nxt.t3);
+    w.v[2] += w.g[0];
+    w.v[5] += w.g[3] - c * (up_own.t1 - up_nxt.t1);
+    w.v[4] += w.g[4] - c * (up_own.t2 - up_nxt.t2);
+    w.v[3] += w.g[5] - c * (up_own.t3 - up_nxt.t3);
+    w.store(p, ny, 1, true);
 }
 
-// Zeroes ghost rows (ROWS) or the ghost columns of the interior rows.
-template <bool ROWS> __global__ void zero_ghosts_kernel(Grid g, double *Ub)
+// One thread per row 2 .. ny-4 and field (blockIdx.y); row 2 only gathers the
+// lower wall face's adjoint from row 3's chains.  blockIdx.y = NFIELD: with
+// mirror y walls, clears what the y pass left of the ghost rows' BYF (except
+// row 2's gathered entries).
+template <int BX> __global__ void xtrans_kernel(Grid g, double *Ub, int clear_rows)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long per_field = ROWS ? 6LL * g.nx : 6LL * (g.ny - 6);
-    if (t >= per_field * NFIELD) return;
-    const int f = (int)(t / per_field);
-    const long long u = t - (long long)f * per_field;
-    int i, j;
-    if (ROWS) {
-        i = (int)(u / 6);
-        const int q = (int)(u - (long long)i * 6);
-        j = q < 3 ? q : g.ny - 6 + q;
-    } else {
-        j = 3 + (int)(u / 6);
-        const int q = (int)(u - (long long)(j - 3) * 6);
-        i = q < 3 ? q : g.nx - 6 + q;
-    }
-    Ub[(long long)f * g.plane + at(g, i, j)] = 0.0;
-}
-
-// x transpose for rows 2 .. ny-4 (row 2 only gathers the lower wall face's
-// adjoint from row 3's chains; every ghost row is zero by now).
-template <int BX> __global__ void xtrans_kernel(Grid g, double *Ub)
-{
-    const int j = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (j > g.ny - 4) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, f = (int)blockIdx.y;
     const long long P = g.plane;
     const int nx = g.nx;
-    auto L = [&](int f, int ii, int jj) -> double & { return Ub[f * P + at(g, ii, jj)]; };
-    if (BX == BC_PERIODIC) {
-        if (j < 3) return;
-#pragma unroll
-        for (int f = 0; f < NFIELD; ++f)
-            for (int q = 0; q < 3; ++q) {
-                L(f, nx - 6 + q, j) += L(f, q, j);
-                L(f, 3 + q, j) += L(f, nx - 3 + q, j);
-            }
+    if (f == NFIELD) {
+        if (!clear_rows || t >= nx) return;
+        double *p = Ub + BYF * P + at(g, t, 0);
+        const bool gathered = BX != BC_PERIODIC && (t == 3 || t == 4 || (t >= nx - 6 && t <= nx - 4));
+        p[0] = p[1] = p[g.ny - 3] = p[g.ny - 2] = p[g.ny - 1] = 0.0;
+        if (!gathered) p[2] = 0.0;
         return;
     }
-    const double c = g.dx / g.dy;
-    auto lower = [&](int row) { return chain_adj(L(BXF, 2, row), L(BXF, 1, row), L(BXF, 0, row)); };
-    auto upper = [&](int row) { return chain_adj(L(BXF, nx - 3, row), L(BXF, nx - 2, row), L(BXF, nx - 1, row)); };
-    const ChainAdj z{0.0, 0.0, 0.0};
-    const ChainAdj lo = j >= 3 ? lower(j) : z, up = j >= 3 ? upper(j) : z;
-    const ChainAdj lo_nxt = lower(j + 1), up_nxt = upper(j + 1);
-    // the chains' bY terms at this row: + from its own chain, - from the next
-    // row's (its j-1), through the copies 2 <- 3 and 1 <- 4
-    L(BYF, 3, j) += c * (lo.t1 - lo_nxt.t1) + c * (lo.t2 - lo_nxt.t2);
-    L(BYF, 4, j) += c * (lo.t3 - lo_nxt.t3);
-    L(BYF, nx - 4, j) -= c * (up.t1 - up_nxt.t1);
-    L(BYF, nx - 5, j) -= c * (up.t2 - up_nxt.t2);
-    L(BYF, nx - 6, j) -= c * (up.t3 - up_nxt.t3);
-    if (j < 3) return;
-    L(BXF, 3, j) += lo.t1;
-    L(BXF, nx - 4, j) += up.t1;
-#pragma unroll
-    for (int f = 0; f < NFIELD; ++f) {
-        if (f == BXF) continue;
-        L(f, 3, j) += L(f, 2, j);
-        L(f, 4, j) += L(f, 1, j);
-        L(f, 5, j) += L(f, 0, j);
-        L(f, nx - 4, j) += L(f, nx - 3, j);
-        L(f, nx - 5, j) += L(f, nx - 2, j);
-        L(f, nx - 6, j) += L(f, nx - 1, j);
+    const int j = 2 + t;
+    if (j > g.ny - 4) return;
+    double *p = Ub + f * P + at(g, 0, j);
+    const long long st = g.pitch;
+    if (BX == BC_PERIODIC) {
+        if (j < 3) return;
+        WallLine w(p, nx, st);
+        w.add_copies(true);
+        w.store(p, nx, st, true);
+        return;
     }
+    if (j < 3 && f != BYF) return;
+    auto B = [&](int i, int row) -> double { return Ub[BXF * P + at(g, i, row)]; };
+    auto lower = [&](int row) { return chain_adj(B(2, row), B(1, row), B(0, row)); };
+    auto upper = [&](int row) { return chain_adj(B(nx - 3, row), B(nx - 2, row), B(nx - 1, row)); };
+    WallLine w(p, nx, st);
+    if (f == BXF) {
+        w.v[0] += chain_adj(w.g[2], w.g[1], w.g[0]).t1;
+        w.v[5] += chain_adj(w.g[3], w.g[4], w.g[5]).t1;
+        w.store(p, nx, st, false);
+        return;
+    }
+    if (f == BYF) {
+        const double c = g.dx / g.dy;
+        const ChainAdj z{0.0, 0.0, 0.0};
+        const ChainAdj lo = j >= 3 ? lower(j) : z, up = j >= 3 ? upper(j) : z;
+        const ChainAdj lo_nxt = lower(j + 1), up_nxt = upper(j + 1);
+        if (j < 3) {
+            // the ghost row's own entries are cleared, not read
+#pragma unroll
+            for (int q = 0; q < 6; ++q) w.v[q] = 0.0;
+        }
+        // the chains' bY terms at this row: + from its own chain, - from the next
+        // row's (its j-1), through the copies 2 <- 3 and 1 <- 4
+        w.v[0] += c * (lo.t1 - lo_nxt.t1) + c * (lo.t2 - lo_nxt.t2);
+        w.v[1] += c * (lo.t3 - lo_nxt.t3);
+        w.v[5] -= c * (up.t1 - up_nxt.t1);
+        w.v[4] -= c * (up.t2 - up_nxt.t2);
+        w.v[3] -= c * (up.t3 - up_nxt.t3);
+        if (j < 3) {
+            p[3 * st] = w.v[0];
+            p[4 * st] = w.v[1];
+            p[(nx - 4) * st] = w.v[5];
+            p[(nx - 5) * st] = w.v[4];
+            p[(nx - 6) * st] = w.v[3];
+            return;
+        }
+    }
+    w.add_copies(false);
+    w.store(p, nx, st, true);
+}
+
+// Clears BXF's ghost columns in the interior rows (blockIdx.y: column).
+__global__ void clear_bx_columns_kernel(Grid g, double *Ub)
+{
+    const int j = 3 + blockIdx.x * blockDim.x + threadIdx.x, q = (int)blockIdx.y;
+    if (j > g.ny - 4) return;
+    Ub[BXF * g.plane + at(g, q < 3 ? q : g.nx - 6 + q, j)] = 0.0;
 }
 
 // Pitched plane -> dense (nx, ny) table.
@@ -397,11 +443,10 @@ int blocks_for(long long n, int threads) { return (int)((n + threads - 1) / thre
 
 void launch_adjoint_stage(const AdjStageArgs &a, cudaStream_t st)
 {
-    const long long n = (long long)a.g.nx * a.g.ny;
     launch_adjoint_prep(a, st);
-    adj_iface_kernel<<<dim3(blocks_for(n, ADJ_THREADS), 2), ADJ_THREADS, 0, st>>>(a);
-    adj_gather_kernel<<<blocks_for(n, ADJ_THREADS), ADJ_THREADS, 0, st>>>(a);
-    adj_center_kernel<<<blocks_for(n, 256), 256, 0, st>>>(a);
+    adj_iface_kernel<<<dim3(IfaceCells::blocks(a.g), 2), IfaceCells::THREADS, 0, st>>>(a);
+    adj_gather_kernel<<<GatherCells::blocks(a.g), GatherCells::THREADS, 0, st>>>(a);
+    adj_center_kernel<<<CenterCells::blocks(a.g), CenterCells::THREADS, 0, st>>>(a);
 }
 
 void launch_boundary_transpose(const Grid &g, double *Ub, cudaStream_t st)
@@ -411,16 +456,20 @@ void launch_boundary_transpose(const Grid &g, double *Ub, cudaStream_t st)
         periodic_transpose_kernel<<<blocks_for(n, 256), 256, 0, st>>>(g, Ub);
         return;
     }
-    if (g.bc_y == BC_PERIODIC)
-        ytrans_kernel<BC_PERIODIC><<<blocks_for(g.nx, 128), 128, 0, st>>>(g, Ub);
+    const dim3 ycols(blocks_for(g.nx, 64), NFIELD);
+    const int along = g.nx > g.ny - 5 ? g.nx : g.ny - 5;
+    const dim3 xrows(blocks_for(along, 64), NFIELD + 1);
+    const int mirror_y = g.bc_y != BC_PERIODIC;
+    if (mirror_y)
+        ytrans_kernel<BC_SYMMETRIC><<<ycols, 64, 0, st>>>(g, Ub);
     else
-        ytrans_kernel<BC_SYMMETRIC><<<blocks_for(g.nx, 128), 128, 0, st>>>(g, Ub);
-    zero_ghosts_kernel<true><<<blocks_for(6LL * g.nx * NFIELD, 256), 256, 0, st>>>(g, Ub);
-    if (g.bc_x == BC_PERIODIC)
-        xtrans_kernel<BC_PERIODIC><<<blocks_for(g.ny - 5, 128), 128, 0, st>>>(g, Ub);
-    else
-        xtrans_kernel<BC_SYMMETRIC><<<blocks_for(g.ny - 5, 128), 128, 0, st>>>(g, Ub);
-    zero_ghosts_kernel<false><<<blocks_for(6LL * (g.ny - 6) * NFIELD, 256), 256, 0, st>>>(g, Ub);
+        ytrans_kernel<BC_PERIODIC><<<ycols, 64, 0, st>>>(g, Ub);
+    if (g.bc_x == BC_PERIODIC) {
+        xtrans_kernel<BC_PERIODIC><<<xrows, 64, 0, st>>>(g, Ub, mirror_y);
+    } else {
+        xtrans_kernel<BC_SYMMETRIC><<<xrows, 64, 0, st>>>(g, Ub, mirror_y);
+        clear_bx_columns_kernel<<<dim3(blocks_for(g.ny - 6, 128), 6), 128, 0, st>>>(g, Ub);
+    }
 }
 
 void launch_plane_to_table(const Grid &g, const double *plane, double *tab, cudaStream_t st)

@@ -7,6 +7,7 @@
 
 #include "adjoint_common.cuh"
 #include "adjoint_core.cuh"
+#include "cell_block.cuh"
 
 namespace rmhd2d {
 
@@ -65,12 +66,13 @@ __device__ void resistive_reverse(const AdjStageArgs &a, int i, int j)
     rj[5 * g.plane] = dbZ;
 }
 
-__global__ void __launch_bounds__(128, 8) adj_prep_kernel(AdjStageArgs a)
+using PrepCells = CellBlock<4>;
+
+__global__ void __launch_bounds__(PrepCells::THREADS, 8) adj_prep_kernel(AdjStageArgs a)
 {
     const Grid &g = a.g;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)g.nx * g.ny) return;
-    const int i = (int)(t / g.ny), j = (int)(t - (long long)i * g.ny);
+    int i, j;
+    if (!PrepCells::cell(g, i, j)) return;
     const long long k = at(g, i, j), P = g.plane;
     if (i >= 1 && i <= g.nx - 2 && j >= 1 && j <= g.ny - 2) {
         const double *W = a.W;
@@ -98,8 +100,7 @@ __global__ void __launch_bounds__(128, 8) adj_prep_kernel(AdjStageArgs a)
 
 void launch_adjoint_prep(const AdjStageArgs &a, cudaStream_t st)
 {
-    const long long n = (long long)a.g.nx * a.g.ny;
-    adj_prep_kernel<<<(int)((n + 127) / 128), 128, 0, st>>>(a);
+    adj_prep_kernel<<<PrepCells::blocks(a.g), PrepCells::THREADS, 0, st>>>(a);
 }
 
 }  // namespace rmhd2d
