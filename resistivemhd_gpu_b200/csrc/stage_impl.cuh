@@ -205,7 +205,8 @@ __device__ __forceinline__ void issue_tile_load(const TileLoad &n, unsigned char
 // and ctl_tile marks the tile that updates the run's control block.
 // Returns false when the bounded wait for the staged tile expired (the CTA
 // must stop).
-template <int STAGE, int SHAPE>
+// IN_LOOP: the caller walks several tiles.
+template <int STAGE, int SHAPE, bool IN_LOOP = false>
 __device__ __forceinline__ bool stage_tile(const StageArgs &a, const TileLoad &load, bool ctl_tile,
                                            unsigned char *smem_raw, uint64_t *bar, uint32_t phase)
 {
@@ -583,6 +584,16 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const TileLoad &l
     // U^n: issue those loads here, so that their latency overlaps the
     // barrier wait of the CTA's slower warps.
     double uo[NFIELD], un_h[6];
+    if (IN_LOOP) {
+        // Only cells of the tile load these.  Set in every turn, or the last
+        // tile's values stay live through the next one's flux phase: the batch
+        // kernels spilled 112 bytes instead of 12 (FP32-bulk) and 328 instead
+        // of 216 (exact), 763 instead of 727 us per step of 24 FP32-bulk runs.
+#pragma unroll
+        for (int f = 0; f < NFIELD; ++f) uo[f] = 0.0;
+#pragma unroll
+        for (int n = 0; n < 6; ++n) un_h[n] = 0.0;
+    }
     if (own) {
 #pragma unroll
         for (int f = 0; f < NFIELD; ++f)
@@ -750,7 +761,7 @@ stage_batch_kernel(const BatchRun *runs, const CUtensorMap *maps, const TileRef 
         const BatchRun &r = runs[tr.run];
         const CUtensorMap *m = maps + (size_t)tr.run * MAPS_PER_RUN;
         const TileLoad load{m + (STAGE - 1), m + 2 + (STAGE - 1), tr.ti, tr.tj, r.eta != nullptr};
-        if (!stage_tile<STAGE, SHAPE>(batch_args<STAGE>(r, parity), load, tr.ti == 0 && tr.tj == 0, smem_raw, bar,
+        if (!stage_tile<STAGE, SHAPE, true>(batch_args<STAGE>(r, parity), load, tr.ti == 0 && tr.tj == 0, smem_raw, bar,
                                       phase))
             return;
         phase ^= 1;
