@@ -224,6 +224,11 @@ template <int BTOP, int QTOP> struct MdDivT {
         ok &= ((~h & 0x000FFFFFu) | ~lo_word(b)) != 0u;
         return rcp_rn_md(b);
     }
+    // x must lie in [2^-BTOP, 2^BTOP)
+    __device__ __forceinline__ void positive(double x)
+    {
+        ok &= (hi_word(x) - ((1023u - BTOP) << 20)) < (2u * BTOP << 20);
+    }
     __device__ __forceinline__ double div(double a, double b, double y)
     {
         const double q = a * y;
@@ -236,9 +241,9 @@ template <int BTOP, int QTOP> struct MdDivT {
     }
 };
 using MdDiv = MdDivT<400, 500>;
-// The HLLD flux's own: with every divisor and quotient below 2^240 (and the
+// The HLLD flux's own: with every divisor and quotient below 2^120 (and the
 // velocities bounded, hlld_flux_sel), no candidate flux can overflow.
-using MdDivFlux = MdDivT<240, 240>;
+using MdDivFlux = MdDivT<120, 120>;
 
 // Division policy with plain IEEE division (the fallback of MdDiv).
 struct IeeeDiv {
@@ -489,29 +494,37 @@ __device__ __forceinline__ void hlld_flux_ieee(const Prim &L, const Prim &R, dou
 // does that after its loop, for the interfaces that asked, so the rare path
 // does not shape the common path's registers).  The conditions:
 //
-// 1. dv.ok: every divisor and quotient is finite and below 2^240.
-// 2. The six velocities are below 1e71.  With 1, the densities (divisors),
-//    |B| (|B|^2 / rho is a quotient), p (p / (gm - 1) is one), SM, pT1 and
-//    the star states are bounded too: v1 and w1 differ from v and w by a
-//    quotient, e2 from e1 by sqrt(rho1) times products of two such values.
-//    No candidate flux, a product of at most three of these (or of e2 and
-//    one), reaches 2^1024, so the reference's F * 0 of the five others is
-//    +-0 and leaves the selected flux bit for bit.
+// 1. dv.ok: every divisor and quotient is finite and below 2^120, and the
+//    star densities lie in [2^-120, 2^120).
+// 2. The six velocities are below 1e35 < 2^120.  With 1, the densities
+//    (divisors), |B| (|B|^2 / rho is a quotient), p (p / (gm - 1) is one),
+//    SM, pT1 and the star states are bounded: v1 and w1 are below 2^121, since
+//    they differ from v and w by a quotient.  The double-star states, whether
+//    formed or not, divide by sqL + sqR >= 2^-59: their numerators are below
+//    2^243, so v2, w2, bY2, bZ2 are below 2^303, and e2, which differs from e1
+//    by sqrt(rho1) times products of two of these, below 2^670.  No candidate
+//    flux, a product of at most three of the outer or star values or of e2 and
+//    SM, reaches 2^1024, so the reference's F * 0 of the others is +-0 and
+//    leaves the selected flux bit for bit.
 // 3. Exactly one region.  SL <= 0 after its clamp, so the left outer state
-//    is never selected.  Under 1, SM, S1L, S1R and SR are not NaN (rho1 < 0
-//    makes sqL + sqR NaN, a divisor) and S1L <= SM <= S1R, since each adds
-//    or subtracts a root; then 0 falls in exactly one of the regions ML, IL,
+//    is never selected.  Under 1, SM, S1L, S1R and SR are not NaN (the roots'
+//    arguments are positive or 0) and S1L <= SM <= S1R, since each adds or
+//    subtracts a root; then 0 falls in exactly one of the regions ML, IL,
 //    IR, and right of S1R; the last is MR for SR > 0, else OR.  SR = 0 with
 //    S1R > 0 selects OR and one more: declined.
+//
+// The double-star states, a sixth of the flux, are formed only by warps with
+// an interface inside them.  Sweeps along a weak normal field have few: the
+// Alfven waves hardly leave the contact.
 __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, double gm, double EPS, double ygm1,
                                               bool gm1_ok, double f[8])
 {
     MdDivFlux dv;
-    dv.ok = gm1_ok;
+    dv.ok = gm1_ok & (EPS >= 0.0);
     const double rhoL = L.rho, uL = L.u, vL = L.v, wL = L.w, bXL = L.bX, bYL = L.bY, bZL = L.bZ, pL = L.p;
     const double rhoR = R.rho, uR = R.u, vR = R.v, wR = R.w, bXR = R.bX, bYR = R.bY, bZR = R.bZ, pR = R.p;
     const double gm1 = gm - 1.0;
-    dv.ok &= (fabs(uL) + fabs(vL) + fabs(wL)) + (fabs(uR) + fabs(vR) + fabs(wR)) < 1e71;
+    dv.ok &= (fabs(uL) + fabs(vL) + fabs(wL)) + (fabs(uR) + fabs(vR) + fabs(wR)) < 1e35;
 
     const double eL = dv.div(pL, gm1, ygm1)
                     + 0.5 * rhoL * (uL * uL + vL * vL + wL * wL)
@@ -569,6 +582,7 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
                               + bXL * ((uL * bXL + vL * bYL + wL * bZL) - vb1L),
                               dLM, yLM);
     const double yr1L = dv.recip(rho1L);
+    dv.positive(rho1L);
     const double S1L = SM - sqrt(dv.div(bXL * bXL, rho1L, yr1L));
     const bool bML = 0.0 < S1L;
     if (bML) {
@@ -591,25 +605,26 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
                               + bXR * ((uR * bXR + vR * bYR + wR * bZR) - vb1R),
                               dRM, yRM);
     const double yr1R = dv.recip(rho1R);
+    dv.positive(rho1R);
     const double S1R = SM + sqrt(dv.div(bXR * bXR, rho1R, yr1R));
     const bool in1R = 0.0 < S1R;   // left of the right Alfven wave
     if (rgt & !in1R) {             // MR
         cr = rho1R; cv = v1R; cw = w1R; cbx = bXR; cby = bY1R; cbz = bZ1R; ce = e1R;
     }
 
-    // double-star states (u2 = SM)
-    const bool bIL = !bML & (0.0 < SM), bI = !bML & in1R;   // IL; IL or IR
-    const double sqL = sqrt(rho1L), sqR = sqrt(rho1R), sqLR = sqrt(rho1L * rho1R);
-    const double sbX = sgn(bXL);
-    const double dsq = sqL + sqR + EPS;
-    const double ysq = dv.recip(dsq);
-    const double v2 = dv.div(sqL * v1L + sqR * v1R + (bY1R - bY1L) * sbX, dsq, ysq);
-    const double w2 = dv.div(sqL * w1L + sqR * w1R + (bZ1R - bZ1L) * sbX, dsq, ysq);
-    const double bY2 = dv.div(sqL * bY1R + sqR * bY1L + sqLR * (v1R - v1L) * sbX, dsq, ysq);
-    const double bZ2 = dv.div(sqL * bZ1R + sqR * bZ1L + sqLR * (w1R - w1L) * sbX, dsq, ysq);
-    const double e2L = e1L - sqL * (vb1L - (SM * bXL + v2 * bY2 + w2 * bZ2)) * sgn(bXL);
-    const double e2R = e1R + sqR * (vb1R - (SM * bXR + v2 * bY2 + w2 * bZ2)) * sgn(bXR);
-    if (bI) {
+    // double-star states (u2 = SM), where the interface lies in them: IL or IR
+    if (!bML & in1R) {
+        const bool bIL = 0.0 < SM;
+        const double sqL = sqrt(rho1L), sqR = sqrt(rho1R), sqLR = sqrt(rho1L * rho1R);
+        const double sbX = sgn(bXL);
+        const double dsq = sqL + sqR + EPS;
+        const double ysq = dv.recip(dsq);
+        const double v2 = dv.div(sqL * v1L + sqR * v1R + (bY1R - bY1L) * sbX, dsq, ysq);
+        const double w2 = dv.div(sqL * w1L + sqR * w1R + (bZ1R - bZ1L) * sbX, dsq, ysq);
+        const double bY2 = dv.div(sqL * bY1R + sqR * bY1L + sqLR * (v1R - v1L) * sbX, dsq, ysq);
+        const double bZ2 = dv.div(sqL * bZ1R + sqR * bZ1L + sqLR * (w1R - w1L) * sbX, dsq, ysq);
+        const double e2L = e1L - sqL * (vb1L - (SM * bXL + v2 * bY2 + w2 * bZ2)) * sgn(bXL);
+        const double e2R = e1R + sqR * (vb1R - (SM * bXR + v2 * bY2 + w2 * bZ2)) * sgn(bXR);
         cr = bIL ? rho1L : rho1R; cv = v2; cw = w2; cbx = bIL ? bXL : bXR;
         cby = bY2; cbz = bZ2; ce = bIL ? e2L : e2R;
     }
