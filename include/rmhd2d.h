@@ -171,7 +171,8 @@ int rmhd2d_run(rmhd2d_solver *s, int nsteps);
    solver's stream; waits and returns the elapsed device time in *ms.
    rmhd2d_profile_step: one step with CUDA events around each of its four
    launches (stage 1, boundary, stage 2, boundary + CFL reduction); waits and
-   returns their device durations in ms[0..3]. */
+   returns their device durations in ms[0..3].  With periodic walls the stages
+   fill the ghosts themselves and the two boundary entries are near 0. */
 int rmhd2d_run_timed(rmhd2d_solver *s, int nsteps, float *ms);
 int rmhd2d_profile_step(rmhd2d_solver *s, float *ms4);
 

@@ -7,6 +7,7 @@
 //
 //   stage 1 (A -> B) ; boundary(B) ; stage 2 (B, A -> A) ; boundary(A) + CFL/NaN
 //
+// (two with periodic walls, whose ghosts the stage kernels write themselves),
 // and the dt of step n+1 is reduced while step n finishes, so no host
 // synchronisation happens inside a step (the reference synchronises on
 // every boundary call and on the dt minimum, resistiveMHD_2D.cu:286-290).
@@ -278,6 +279,7 @@ void enqueue_step_between(rmhd2d_solver *s, int parity, const double *un, const 
     s->mirrored = false;
     StageArgs a{};
     a.dt_in = dt_in;
+    a.wrap = wraps(s->g);
     a.g = s->g;
     a.eta = s->eta;
     a.row2 = s->g.bc_x == BC_SYMMETRIC ? s->row2 : nullptr;
@@ -289,12 +291,12 @@ void enqueue_step_between(rmhd2d_solver *s, int parity, const double *un, const 
     a.dt_log = dt_log;
     launch_planned(s, 1, map_un, a);
     a.dt_log = nullptr;
-    launch_boundary(s->g, ustar, s->row2, nullptr, 0, s->stream);
+    if (!a.wrap) launch_boundary(s->g, ustar, s->row2, nullptr, 0, s->stream);
     a.src = ustar;
     a.un = un;
     a.dst = dst;
     launch_planned(s, 2, map_ustar, a);
-    launch_boundary(s->g, dst, s->row2, s->ctl, parity ^ 1, s->stream);
+    if (!a.wrap) launch_boundary(s->g, dst, s->row2, s->ctl, parity ^ 1, s->stream);
 }
 
 // dt_log: stage 1 also writes the step's dt there (a recorded run); dt_in:
@@ -333,6 +335,7 @@ void enqueue_step(rmhd2d_solver *s, int parity, double *dt_log = nullptr, const 
     a.ctl = s->ctl;
     a.parity = parity;
     a.dt_in = dt_in;
+    a.wrap = wraps(s->g);
     // stage 1: U^n (A) -> U* (B)
     a.src = s->A;
     a.un = s->A;
@@ -340,13 +343,14 @@ void enqueue_step(rmhd2d_solver *s, int parity, double *dt_log = nullptr, const 
     a.dt_log = dt_log;
     launch_planned(s, 1, &s->mapA[stage_plan(s, 1)], a);
     a.dt_log = nullptr;
-    launch_boundary(s->g, s->B, s->row2, nullptr, 0, s->stream);
+    if (!a.wrap) launch_boundary(s->g, s->B, s->row2, nullptr, 0, s->stream);
     // stage 2: (U*, U^n) -> U^{n+1} in A
     a.src = s->B;
     a.un = s->A;
     a.dst = s->A;
+    if (a.wrap) a.mirror = mirror;
     launch_planned(s, 2, &s->mapB[stage_plan(s, 2)], a);
-    launch_boundary_mirrored(s->g, s->A, s->row2, s->ctl, parity ^ 1, mirror, s->stream);
+    if (!a.wrap) launch_boundary_mirrored(s->g, s->A, s->row2, s->ctl, parity ^ 1, mirror, s->stream);
 }
 
 int upload_from_device_aos(rmhd2d_solver *s, const double *aos_dev, int apply_boundary)
@@ -812,16 +816,17 @@ int rmhd2d_profile_step(rmhd2d_solver *s, float *ms4)
     a.row2 = s->g.bc_x == BC_SYMMETRIC ? s->row2 : nullptr;
     a.ctl = s->ctl;
     a.parity = parity;
+    a.wrap = wraps(s->g);
     CK(cudaEventRecord(ev[0], s->stream));
     a.src = s->A; a.un = s->A; a.dst = s->B;
     launch_planned(s, 1, &s->mapA[stage_plan(s, 1)], a);
     CK(cudaEventRecord(ev[1], s->stream));
-    launch_boundary(s->g, s->B, s->row2, nullptr, 0, s->stream);
+    if (!a.wrap) launch_boundary(s->g, s->B, s->row2, nullptr, 0, s->stream);
     CK(cudaEventRecord(ev[2], s->stream));
     a.src = s->B; a.un = s->A; a.dst = s->A;
     launch_planned(s, 2, &s->mapB[stage_plan(s, 2)], a);
     CK(cudaEventRecord(ev[3], s->stream));
-    launch_boundary(s->g, s->A, s->row2, s->ctl, parity ^ 1, s->stream);
+    if (!a.wrap) launch_boundary(s->g, s->A, s->row2, s->ctl, parity ^ 1, s->stream);
     CK(cudaEventRecord(ev[4], s->stream));
     CK(cudaGetLastError());
     CK(cudaEventSynchronize(ev[4]));
@@ -1069,6 +1074,7 @@ struct rmhd2d_batch {
     int parity = 0;
     long long steps = 0;
     long long max_ghost = 0;
+    bool all_wrap = true;                     // every run's stage kernels write their ghosts themselves
     BatchRun *d_runs = nullptr;
     CUtensorMap *d_maps = nullptr;            // MAPS_PER_RUN per run, for the current shape
     TileRef *d_tiles[2] = {nullptr, nullptr}; // stage 1 / stage 2 tile tables
@@ -1119,6 +1125,7 @@ int batch_build(rmhd2d_batch *b)
     std::vector<CUtensorMap> maps((size_t)n * MAPS_PER_RUN);
     std::vector<TileRef> tiles[2];
     b->max_ghost = 0;
+    b->all_wrap = true;
     for (int r = 0; r < n; ++r) {
         rmhd2d_solver *s = b->runs[r];
         if (!s->has_state) return bfail(b, RMHD2D_ERR_STATE, "run " + std::to_string(r) + " has no state");
@@ -1129,6 +1136,7 @@ int batch_build(rmhd2d_batch *b)
         maps[(size_t)r * MAPS_PER_RUN + 3] = s->mapE2[b->shape];
         const long long ng = 6LL * s->g.ny + 6LL * (s->g.nx - 6);
         b->max_ghost = ng > b->max_ghost ? ng : b->max_ghost;
+        b->all_wrap = b->all_wrap && wraps(s->g);
         for (int st = 1; st <= 2; ++st) {
             const int ti = stage_ti(st, b->shape), tj = shape_tj(b->shape);
             const int nti = (s->g.nx - 2 * HALO + ti - 1) / ti, ntj = (s->g.ny - 2 * HALO + tj - 1) / tj;
@@ -1166,9 +1174,9 @@ void batch_enqueue_step(rmhd2d_batch *b, int parity)
     const int n = (int)b->runs.size();
     const int ctas = b->nsm * b->ctas_per_sm;
     launch(1, b->shape, b->d_runs, b->d_maps, b->d_tiles[0], b->ntiles[0], ctas, parity, b->stream);
-    launch_boundary_batch(b->d_runs, n, b->max_ghost, 0, 0, b->stream);
+    if (!b->all_wrap) launch_boundary_batch(b->d_runs, n, b->max_ghost, 0, 0, b->stream);
     launch(2, b->shape, b->d_runs, b->d_maps, b->d_tiles[1], b->ntiles[1], ctas, parity, b->stream);
-    launch_boundary_batch(b->d_runs, n, b->max_ghost, 1, parity ^ 1, b->stream);
+    if (!b->all_wrap) launch_boundary_batch(b->d_runs, n, b->max_ghost, 1, parity ^ 1, b->stream);
 }
 
 void batch_advance(rmhd2d_batch *b, int nsteps)

@@ -45,7 +45,15 @@ struct StageArgs {
     int parity;          // step parity: dt from ctl->amax[parity]
     double *dt_log;      // stage 1, or nullptr: the step's dt is also written here (a recorded run)
     const double *dt_in; // or nullptr: the step's dt is read from here (a replayed run), not reduced
+    int wrap;            // both walls periodic: the update also writes its cells' ghost images (no ghost fill follows)
+    Control *mirror;     // stage 2 with wrap, or nullptr: the launch leaves the control block there (host memory)
 };
+
+// Whether the stage kernels write a grid's ghost cells themselves.
+__host__ __device__ __forceinline__ bool wraps(const Grid &g)
+{
+    return g.bc_x == BC_PERIODIC && g.bc_y == BC_PERIODIC && !g.x_halo;
+}
 
 // One set of launchers per variant (stage_exact.cu, stage_fast.cu, stage_bulk32.cu).
 // Sweep of the stage kernel's flux phase (true: x sweep), as a compile-time

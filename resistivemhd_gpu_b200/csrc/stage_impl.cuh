@@ -170,6 +170,49 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t phase)
     return false;
 }
 
+// Writes a cell's new values v, and under periodic walls (wrap) its ghost
+// images (boundary.cu:4-141): ghost c < 3 holds cell c + n - 6, ghost c >= n - 3
+// cell c - (n - 6).  This spares the step's two ghost-fill launches, about 4 us
+// each (exact, 128 x 128: 22.6 -> 17.4 us per step).
+__device__ __forceinline__ void store_cell(const Grid &g, double *dst, int i, int j, bool wrap, const double v[NFIELD])
+{
+    double *p = dst + (long long)i * g.pitch + j;
+#pragma unroll
+    for (int f = 0; f < NFIELD; ++f) p[f * g.plane] = v[f];
+    if (!wrap) return;
+    const int px = g.nx - 2 * HALO, py = g.ny - 2 * HALO;
+    const int di = i < 2 * HALO ? px : i >= px ? -px : 0, dj = j < 2 * HALO ? py : j >= py ? -py : 0;
+    const long long oi = (long long)di * g.pitch;
+    if (dj) {
+#pragma unroll
+        for (int f = 0; f < NFIELD; ++f) p[f * g.plane + dj] = v[f];
+    }
+    if (di) {
+#pragma unroll
+        for (int f = 0; f < NFIELD; ++f) p[f * g.plane + oi] = v[f];
+        if (dj) {
+#pragma unroll
+            for (int f = 0; f < NFIELD; ++f) p[f * g.plane + oi + dj] = v[f];
+        }
+    }
+}
+
+// Leaves the control block in host memory when the launch's last CTA calls
+// this (one thread per CTA, after its own writes to the control block).
+__device__ __forceinline__ void mirror_control(Control *ctl, Control *mirror)
+{
+    __threadfence();
+    const unsigned long long ctas = (unsigned long long)gridDim.x * gridDim.y;
+    if (atomicAdd(&ctl->ghost_blocks, 1ull) != ctas - 1) return;
+    __threadfence();
+    static_assert(sizeof(Control) % 8 == 0, "copied by words");
+#pragma unroll
+    for (int w = 0; w < (int)(sizeof(Control) / 8); ++w)
+        reinterpret_cast<unsigned long long *>(mirror)[w] =
+            __ldcg(reinterpret_cast<const unsigned long long *>(ctl) + w);
+    ctl->ghost_blocks = 0ull;
+}
+
 // A tile's staging: its run's tensor maps, its tile index, and whether the
 // run has an eta table.
 struct TileLoad {
@@ -641,14 +684,16 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const TileLoad &l
     if (STAGE == 1) {
         if (own) {
             // oneStepFirstFunctor (resistiveMHD_2D.cu:53-86)
+            double nv[NFIELD];
 #pragma unroll
             for (int n = 0; n < 6; ++n)
-                a.dst[fld[n] * PL + k] = uo[fld[n]] - dtdx * dF(n) - dtdy * dG(n);
+                nv[fld[n]] = uo[fld[n]] - dtdx * dF(n) - dtdy * dG(n);
             // CT_kernel (ct.cu:44-59) with the EMF of this stage
             const double ez_c = corner_ez(li + 1, lj + 1), ez_w = corner_ez(li + 1, lj);
             const double ez_s = corner_ez(li, lj + 1);
-            a.dst[BXF * PL + k] = uo[BXF] - dtdy * (ez_c - ez_w);
-            a.dst[BYF * PL + k] = uo[BYF] + dtdx * (ez_c - ez_s);
+            nv[BXF] = uo[BXF] - dtdy * (ez_c - ez_w);
+            nv[BYF] = uo[BYF] + dtdx * (ez_c - ez_s);
+            store_cell(g, a.dst, i, j, a.wrap, nv);
             // Symmetric boundaries read the CT'd face bY at j = 2 (the lower
             // wall face) before replacing it (TS boundary.cu:57-88).
             if (a.row2 && j0 == HALO && lj == 0) {
@@ -670,8 +715,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const TileLoad &l
             }
             nv[BXF] = uo[BXF];
             nv[BYF] = uo[BYF];
-#pragma unroll
-            for (int n = 0; n < 8; ++n) a.dst[n * PL + k] = nv[n];
+            store_cell(g, a.dst, i, j, a.wrap, nv);
         }
         // next step's CFL rate and the crash flag over the interior
         // (ghosts are reduced by the boundary kernel)
@@ -689,6 +733,8 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const TileLoad &l
 #endif
             bits = rate_bits(r);
             nan_e = nv[EN] != nv[EN];
+            // the image of this cell is cell 0, the reductions' first candidate
+            if (a.wrap && r != r && i == g.nx - 2 * HALO && j == g.ny - 2 * HALO) a.ctl->first_nan[a.parity ^ 1] = 1;
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -704,6 +750,7 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const TileLoad &l
             for (int w = 0; w < T::THREADS / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
             atomicMax(&a.ctl->amax[a.parity ^ 1], m);
             if (any_nan) atomicExch(&a.ctl->crashed, 1);
+            if (a.mirror) mirror_control(a.ctl, a.mirror);
         }
     }
     return true;
@@ -742,6 +789,7 @@ __device__ __forceinline__ StageArgs batch_args(const BatchRun &r, int parity)
     a.row2 = r.g.bc_x == BC_SYMMETRIC ? r.row2 : nullptr;
     a.ctl = r.ctl;
     a.parity = parity;
+    a.wrap = wraps(r.g);
     return a;
 }
 
