@@ -132,7 +132,10 @@ __device__ __forceinline__ void gather_sweep(const AdjStageArgs &a, int dir, int
     for (int s = 0; s < 8; ++s) nat_bar[sweep_field(dir, s)] += cb[s];
 }
 
-__global__ void __launch_bounds__(GatherCells::THREADS, 3) adj_gather_kernel(AdjStageArgs a)
+// Bound by the latency of its 120 loads per cell: at 128 registers (two blocks
+// per SM) more of them are in flight than at 80 (three): 130 x 96 x 36 steps and
+// their reverse 4.77 -> 4.57 ms, 150 x 90 4.96 -> 4.82, 512 x 512 22.7 -> 22.5.
+__global__ void __launch_bounds__(GatherCells::THREADS, 2) adj_gather_kernel(AdjStageArgs a)
 {
     const Grid &g = a.g;
     int i, j;
@@ -202,23 +205,21 @@ __global__ void __launch_bounds__(256) adj_center_kernel(AdjStageArgs a)
 // image, so no two threads touch the same entry.
 __global__ void periodic_transpose_kernel(Grid g, double *Ub)
 {
-    const long long nrow = 6LL * (g.nx - 6);    // rows 3..5 and ny-6..ny-4, interior columns
-    const long long ncol = 6LL * (g.ny - 12);   // columns 3..5 and nx-6..nx-4, rows 6..ny-7
-    const long long per_field = nrow + ncol;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= per_field * NFIELD) return;
-    const int f = (int)(t / per_field);
-    long long u = t - (long long)f * per_field;
+    const unsigned nrow = 6u * (unsigned)(g.nx - 6);    // rows 3..5 and ny-6..ny-4, interior columns
+    const unsigned ncol = 6u * (unsigned)(g.ny - 12);   // columns 3..5 and nx-6..nx-4, rows 6..ny-7
+    unsigned u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= nrow + ncol) return;
+    const int f = (int)blockIdx.y;
     int I, J;
     if (u < nrow) {
-        const int r = (int)(u / (g.nx - 6));
-        I = 3 + (int)(u - (long long)r * (g.nx - 6));
-        J = r < 3 ? 3 + r : g.ny - 9 + r;
+        const unsigned r = u / (unsigned)(g.nx - 6);
+        I = 3 + (int)(u - r * (unsigned)(g.nx - 6));
+        J = (int)r + (r < 3 ? 3 : g.ny - 9);
     } else {
         u -= nrow;
-        const int c = (int)(u / (g.ny - 12));
-        J = 6 + (int)(u - (long long)c * (g.ny - 12));
-        I = c < 3 ? 3 + c : g.nx - 9 + c;
+        const unsigned c = u / (unsigned)(g.ny - 12);
+        J = 6 + (int)(u - c * (unsigned)(g.ny - 12));
+        I = (int)c + (c < 3 ? 3 : g.nx - 9);
     }
     const int Ig = I < 6 ? I + g.nx - 6 : (I >= g.nx - 6 ? I - (g.nx - 6) : -1);
     const int Jg = J < 6 ? J + g.ny - 6 : (J >= g.ny - 6 ? J - (g.ny - 6) : -1);
@@ -452,8 +453,8 @@ void launch_adjoint_stage(const AdjStageArgs &a, cudaStream_t st)
 void launch_boundary_transpose(const Grid &g, double *Ub, cudaStream_t st)
 {
     if (g.bc_x == BC_PERIODIC && g.bc_y == BC_PERIODIC) {
-        const long long n = (6LL * (g.nx - 6) + 6LL * (g.ny - 12)) * NFIELD;
-        periodic_transpose_kernel<<<blocks_for(n, 256), 256, 0, st>>>(g, Ub);
+        const long long n = 6LL * (g.nx - 6) + 6LL * (g.ny - 12);
+        periodic_transpose_kernel<<<dim3(blocks_for(n, 128), NFIELD), 128, 0, st>>>(g, Ub);
         return;
     }
     const dim3 ycols(blocks_for(g.nx, 64), NFIELD);
