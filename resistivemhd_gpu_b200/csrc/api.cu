@@ -548,7 +548,7 @@ int rmhd2d_create(const rmhd2d_config *cfg, rmhd2d_solver **out)
     const size_t state_bytes = (size_t)g.plane * NFIELD * sizeof(double);
     if (cudaMalloc(&s->A, state_bytes) != cudaSuccess || cudaMalloc(&s->B, state_bytes) != cudaSuccess ||
         cudaMalloc(&s->row2, (size_t)g.nx * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&s->ctl, sizeof(Control)) != cudaSuccess ||
+        cudaMalloc(&s->ctl, sizeof(ControlSlot)) != cudaSuccess ||
         cudaMallocHost(&s->ctl_host, sizeof(Control)) != cudaSuccess)
         return bail(RMHD2D_ERR_CUDA, "device allocation failed");
     // Every clear goes on the solver's stream, which does not synchronise
@@ -565,7 +565,7 @@ int rmhd2d_create(const rmhd2d_config *cfg, rmhd2d_solver **out)
     if (cudaMemsetAsync(s->A, 0, state_bytes, s->stream) != cudaSuccess ||
         cudaMemsetAsync(s->B, 0, state_bytes, s->stream) != cudaSuccess ||
         cudaMemsetAsync(s->row2, 0, (size_t)g.nx * sizeof(double), s->stream) != cudaSuccess ||
-        cudaMemsetAsync(s->ctl, 0, sizeof(Control), s->stream) != cudaSuccess ||
+        cudaMemsetAsync(s->ctl, 0, sizeof(ControlSlot), s->stream) != cudaSuccess ||
         cudaStreamSynchronize(s->stream) != cudaSuccess)
         return bail(RMHD2D_ERR_CUDA, "device memset failed");
     for (int sh = 0; sh < NSHAPE_ALL; ++sh)

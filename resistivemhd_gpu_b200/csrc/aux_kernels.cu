@@ -338,14 +338,15 @@ boundary_kernel(Grid g, double *s, const double *row2, Control *ctl, int slot, C
     if (!mirror) return;
     // (the block's writes to the control block are all lane 0's)
     __threadfence();
-    const bool last = lane == 0 && atomicAdd(&ctl->ghost_blocks, 1ull) == gridDim.x - 1ull;
+    unsigned long long *done = &reinterpret_cast<ControlSlot *>(ctl)->blocks_done;
+    const bool last = lane == 0 && atomicAdd(done, 1ull) == gridDim.x - 1ull;
     if (!__any_sync(0xffffffffu, last)) return;
     __threadfence();
     static_assert(sizeof(Control) % 8 == 0 && sizeof(Control) / 8 <= 32, "one word per lane");
     if (lane < (int)(sizeof(Control) / 8))
         reinterpret_cast<unsigned long long *>(mirror)[lane] =
             __ldcg(reinterpret_cast<const unsigned long long *>(ctl) + lane);
-    if (last) ctl->ghost_blocks = 0ull;
+    if (last) *done = 0ull;
 }
 
 // Every ghost cell of every run of a batch (blockIdx.y = run); `which`

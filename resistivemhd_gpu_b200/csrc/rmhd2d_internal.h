@@ -41,7 +41,14 @@ struct Control {
     int error;                   // kernel-side error code (bounded wait expired, ...)
     double dt_fixed;             // dt of the next step when use_fixed_dt is set
     int use_fixed_dt;            // 1: steps take dt_fixed instead of the CFL dt (frozen-dt runs)
-    unsigned long long ghost_blocks;  // blocks of the step's last ghost fill that have finished (back to 0 after it)
+};
+
+// A solver's control block on the device, with the count behind it that the
+// queries do not read back: the blocks of a step's last launch that have
+// finished, back to 0 when the last of them leaves the mirror.
+struct ControlSlot {
+    Control c;
+    unsigned long long blocks_done;
 };
 
 enum KernelError { KERR_NONE = 0, KERR_TMA_TIMEOUT = 1 };

@@ -203,14 +203,15 @@ __device__ __forceinline__ void mirror_control(Control *ctl, Control *mirror)
 {
     __threadfence();
     const unsigned long long ctas = (unsigned long long)gridDim.x * gridDim.y;
-    if (atomicAdd(&ctl->ghost_blocks, 1ull) != ctas - 1) return;
+    unsigned long long *done = &reinterpret_cast<ControlSlot *>(ctl)->blocks_done;
+    if (atomicAdd(done, 1ull) != ctas - 1) return;
     __threadfence();
     static_assert(sizeof(Control) % 8 == 0, "copied by words");
 #pragma unroll
     for (int w = 0; w < (int)(sizeof(Control) / 8); ++w)
         reinterpret_cast<unsigned long long *>(mirror)[w] =
             __ldcg(reinterpret_cast<const unsigned long long *>(ctl) + w);
-    ctl->ghost_blocks = 0ull;
+    *done = 0ull;
 }
 
 // A tile's staging: its run's tensor maps, its tile index, and whether the
