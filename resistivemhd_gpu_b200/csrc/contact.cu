@@ -8,9 +8,9 @@
 // and dt:
 //   begin        dt (CFL or the fixed dt), the control block's step fields
 //   flux         F, G of the cell-centred U^n (HLLD, MUSCL, resistive hook)
-//   ref (old)    per-cell reference EMF u bY - v bX - eta jZ of U^n with the
-//                face B that shift + back-to-face leave (smoothed)
-//   update 1     U* = U^n - dt div(F, G) for all 8 fields (smoothed face B)
+//   update 1     U* = U^n - dt div(F, G) for all 8 fields, with the face B that
+//                shift + back-to-face leave (smoothed), and from the same reads
+//                ref (old), the per-cell reference EMF u bY - v bX - eta jZ of U^n
 //   boundary     U*
 //   flux         F, G of the cell-centred U*
 //   update 2     C = (U^n + U* - dt div(F, G)) / 2 (both with smoothed face B)
