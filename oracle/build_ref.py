@@ -156,7 +156,7 @@ def build_mc(verbose=True) -> bool:
 
 def build(which=("gpu", "cpu"), verbose=True) -> bool:
     """Build the reference binaries; returns False when the reference is absent."""
-    if not REF_ROOT.is_dir():
+    if not all((REF_ROOT / rel).is_dir() for rel in LIBS.values()):
         if verbose:
             print(f"[build_ref] reference tree {REF_ROOT} absent; using prebuilt oracle/_ref", file=sys.stderr)
         return False
