@@ -551,6 +551,7 @@ int rmhd2d_create(const rmhd2d_config *cfg, rmhd2d_solver **out)
         cudaMalloc(&s->ctl, sizeof(ControlSlot)) != cudaSuccess ||
         cudaMallocHost(&s->ctl_host, sizeof(Control)) != cudaSuccess)
         return bail(RMHD2D_ERR_CUDA, "device allocation failed");
+    *s->ctl_host = Control{};
     // Every clear goes on the solver's stream, which does not synchronise
     // with the legacy default stream (cudaStreamNonBlocking): a plain
     // cudaMemset there could still be running when set_state's copy lands

@@ -198,7 +198,9 @@ __device__ __forceinline__ void store_cell(const Grid &g, double *dst, int i, in
 }
 
 // Leaves the control block in host memory when the launch's last CTA calls
-// this (one thread per CTA, after its own writes to the control block).
+// this: one thread of every CTA, after the CTA's own writes to the control
+// block.  A CTA that gave up its wait counts too: the host reads the error
+// from the mirror, and the next step counts from 0.
 __device__ __forceinline__ void mirror_control(Control *ctl, Control *mirror)
 {
     __threadfence();
@@ -751,7 +753,6 @@ __device__ __forceinline__ bool stage_tile(const StageArgs &a, const TileLoad &l
             for (int w = 0; w < T::THREADS / 32; ++w) m = wmax[w] > m ? wmax[w] : m;
             atomicMax(&a.ctl->amax[a.parity ^ 1], m);
             if (any_nan) atomicExch(&a.ctl->crashed, 1);
-            if (a.mirror) mirror_control(a.ctl, a.mirror);
         }
     }
     return true;
@@ -775,6 +776,8 @@ stage_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ C
     init_tile_barrier(bar);
     const TileLoad load{&tmap, &emap, (int)blockIdx.y, (int)blockIdx.x, a.eta != nullptr};
     stage_tile<STAGE, SHAPE>(a, load, blockIdx.x == 0 && blockIdx.y == 0, smem_raw, bar, 0);
+    // (all that a CTA writes to the control block lies before a barrier or is thread 0's)
+    if (STAGE == 2 && a.mirror && threadIdx.x == 0) mirror_control(a.ctl, a.mirror);
 }
 
 // The stage arguments of one run of a batch.
