@@ -51,7 +51,7 @@ struct rmhd2d_solver {
     // The last work enqueued that changes the control block was a one-step
     // graph, which leaves the control block in ctl_host itself.
     bool mirrored = false;
-    bool captured = false;       // a caller has captured a step: its replays change the control block unseen
+    bool captured = false;       // a caller has captured such work: its replays change the control block unseen
     // per tile shape: stage-1 source A, stage-2 source B, eta plane with the
     // stage-1 and stage-2 boxes
     CUtensorMap mapA[NSHAPE_ALL]{}, mapB[NSHAPE_ALL]{}, mapE1[NSHAPE_ALL]{}, mapE2[NSHAPE_ALL]{};
@@ -174,11 +174,22 @@ int sync_and_check(rmhd2d_solver *s)
     return RMHD2D_OK;
 }
 
+// To be called where work that changes the control block is enqueued.  While
+// the caller captures the stream, that work runs when the caller replays it,
+// also behind a later step's mirror: from then on every query copies the
+// control block.
+void control_changes(rmhd2d_solver *s)
+{
+    s->mirrored = false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) s->captured = true;
+}
+
 // Re-reduces the CFL rate and crash flag of the current state into slot
 // `parity` (after a state change outside a step).
 int refresh_rate(rmhd2d_solver *s)
 {
-    s->mirrored = false;
+    control_changes(s);
     CK(cudaMemsetAsync(&s->ctl->amax[s->parity], 0, sizeof(unsigned long long), s->stream));
     CK(cudaMemsetAsync(&s->ctl->first_nan[s->parity], 0, sizeof(int), s->stream));
     CK(cudaMemsetAsync(&s->ctl->crashed, 0, sizeof(int), s->stream));
@@ -276,7 +287,7 @@ void launch_planned(rmhd2d_solver *s, int stage, const CUtensorMap *map, const S
 void enqueue_step_between(rmhd2d_solver *s, int parity, const double *un, const CUtensorMap *map_un, double *ustar,
                           const CUtensorMap *map_ustar, double *dst, double *dt_log, const double *dt_in)
 {
-    s->mirrored = false;
+    control_changes(s);
     StageArgs a{};
     a.dt_in = dt_in;
     a.wrap = wraps(s->g);
@@ -306,7 +317,7 @@ void enqueue_step_between(rmhd2d_solver *s, int parity, const double *un, const 
 void enqueue_step(rmhd2d_solver *s, int parity, double *dt_log = nullptr, const double *dt_in = nullptr,
                   Control *mirror = nullptr)
 {
-    s->mirrored = false;
+    control_changes(s);
     if (s->contact) {
         const size_t P = (size_t)s->g.plane;
         ContactStep c{};
@@ -386,7 +397,7 @@ void free_adjoint(AdjointWork *w)
 // Sets or clears Control::use_fixed_dt in stream order.
 int set_fixed_dt_mode(rmhd2d_solver *s, int on)
 {
-    s->mirrored = false;
+    control_changes(s);
     static const int kOn = 1, kOff = 0;
     CK(cudaMemcpyAsync(&s->ctl->use_fixed_dt, on ? &kOn : &kOff, sizeof(int), cudaMemcpyHostToDevice, s->stream));
     return RMHD2D_OK;
@@ -698,10 +709,12 @@ int rmhd2d_calculate_dt(rmhd2d_solver *s, double *dt)
 static int capture_steps(rmhd2d_solver *s, int parity, int nsteps, cudaGraphExec_t *ge)
 {
     cudaGraph_t graph = nullptr;
+    const bool captured = s->captured;   // by the caller: this capture is the library's own
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     // a one-step graph ends with the control block in the host's mirror
     for (int n = 0; n < nsteps; ++n)
         enqueue_step(s, parity ^ (n & 1), nullptr, nullptr, nsteps == 1 ? s->ctl_host : nullptr);
+    s->captured = captured;
     cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
     if (e != cudaSuccess) return fail(s, RMHD2D_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     e = cudaGraphInstantiate(ge, graph, 0);
@@ -741,7 +754,6 @@ int rmhd2d_step_rk2(rmhd2d_solver *s)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s->stream, &cap));
     if (cap != cudaStreamCaptureStatusNone) {
-        s->captured = true;
         enqueue_step(s, s->parity);
         CK(cudaGetLastError());
     } else {
@@ -769,7 +781,7 @@ int rmhd2d_run(rmhd2d_solver *s, int nsteps)
         if (rc) return rc;
     }
     while (nsteps >= 2) {
-        s->mirrored = false;
+        s->mirrored = false;   // (the runtime refuses a graph launch under a caller's capture)
         CK(cudaGraphLaunch(s->graph2[s->parity], s->stream));
         s->steps += 2;
         nsteps -= 2;
@@ -810,7 +822,7 @@ int rmhd2d_profile_step(rmhd2d_solver *s, float *ms4)
         ev[n] = sev[n].e;
     }
     const int parity = s->parity;
-    s->mirrored = false;
+    control_changes(s);
     StageArgs a{};
     a.g = s->g;
     a.eta = s->eta;
@@ -988,7 +1000,7 @@ static int snapshot_take(rmhd2d_solver *s, Snapshot &sn)
 static int snapshot_restore(rmhd2d_solver *s, Snapshot &sn)
 {
     const size_t bytes = (size_t)s->g.plane * NFIELD * sizeof(double);
-    s->mirrored = false;
+    control_changes(s);
     CK(cudaMemcpyAsync(s->A, sn.A, bytes, cudaMemcpyDeviceToDevice, s->stream));
     CK(cudaMemcpyAsync(s->ctl, &sn.ctl, sizeof(Control), cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
@@ -1558,7 +1570,7 @@ int rmhd2d_slab_stage(rmhd2d_solver *s, int stage)
     if (stage != 1 && stage != 2) return fail(s, RMHD2D_ERR_INVALID, "stage must be 1 or 2");
     if (!s->has_state) return fail(s, RMHD2D_ERR_STATE, "no state set");
     CK(cudaSetDevice(s->device));
-    s->mirrored = false;
+    control_changes(s);
     StageArgs a{};
     a.g = s->g;
     a.eta = s->eta;
@@ -1587,7 +1599,7 @@ int rmhd2d_slab_fill(rmhd2d_solver *s, int which)
     if (which < 0 || which > 2) return fail(s, RMHD2D_ERR_INVALID, "which must be 0, 1 or 2");
     if (!s->has_state) return fail(s, RMHD2D_ERR_STATE, "no state set");
     CK(cudaSetDevice(s->device));
-    s->mirrored = false;
+    control_changes(s);
     if (which == 0) {
         if (s->g.bc_x == BC_SYMMETRIC) launch_snapshot_row2(s->g, s->A, s->row2, s->stream);
         launch_boundary(s->g, s->A, s->row2, nullptr, 0, s->stream);
@@ -1618,7 +1630,7 @@ int rmhd2d_slab_get_words(rmhd2d_solver *s, long long *dev_words)
     CK(cudaSetDevice(s->device));
     // the domain's ghost column 0 of a periodic-x decomposition sits in the
     // first slab's low halo, which its neighbour has just filled
-    s->mirrored = false;
+    control_changes(s);
     if ((s->slab & RMHD2D_SLAB_ORIGIN) && (s->g.x_halo & 1))
         launch_slab_origin_column(s->g, s->A, s->ctl, s->parity, s->stream);
     launch_slab_words(s->ctl, s->parity, dev_words, 1, s->stream);
@@ -1631,7 +1643,7 @@ int rmhd2d_slab_set_words(rmhd2d_solver *s, const long long *dev_words)
     if (!s || !dev_words) return fail(s, RMHD2D_ERR_INVALID, "null argument");
     if (!(s->slab & SLAB_CREATED)) return fail(s, RMHD2D_ERR_STATE, "not a slab (rmhd2d_create_slab)");
     CK(cudaSetDevice(s->device));
-    s->mirrored = false;
+    control_changes(s);
     launch_slab_words(s->ctl, s->parity, const_cast<long long *>(dev_words), 0, s->stream);
     CK(cudaGetLastError());
     return RMHD2D_OK;
