@@ -207,14 +207,19 @@ int rmhd2d_write_snapshot(const char *path, const double *host_state, int nx, in
    2: 16x32 / 18x32 with 640 threads, 1 CTA per SM (fewer redundant ring
    fluxes per cell); 3: 8x64 / 8x64 with 512 threads, 1 CTA per SM (128
    registers per thread); 4: 8x32 / 8x32 and 5: 6x32 / 7x32 with 256
-   threads, 3 CTAs per SM.
-   Each stage has its own shape: rmhd2d_set_tile_shape
-   sets both, rmhd2d_set_stage_shapes each, rmhd2d_get_tile_shape returns
-   stage 1's.  rmhd2d_autotune times trial_steps steps with each shape (CUDA
-   events around each stage's launch; the state is restored afterwards),
-   keeps the fastest shape of each stage, and returns stage 1's;
-   rmhd2d_get_tuning returns the median ms of each stage with each shape (up
-   to max entries; *n = the number of shapes tried, 0 before any autotune).
+   threads, 3 CTAs per SM; 6: 4x16 / 4x16 with 192 threads, one interface
+   each, 2 CTAs per SM (for grids too small to fill the SMs).
+   A solver starts with shape 6 while the grid has at most 296 such tiles
+   (two per SM), with 4 and 5 (FP32-bulk: 4 and 4) from 2^18 interior cells,
+   and with shape 0 between.  Each stage has its own shape:
+   rmhd2d_set_tile_shape sets both, rmhd2d_set_stage_shapes each,
+   rmhd2d_get_tile_shape returns stage 1's, rmhd2d_get_stage_shapes both, as
+   the next step runs them.  rmhd2d_autotune times trial_steps steps with
+   each shape (6 on the grids that start with it; CUDA events around each
+   stage's launch; the state is restored afterwards), keeps the fastest shape
+   of each stage, and returns stage 1's; rmhd2d_get_tuning returns the median
+   ms of each stage with each shape (up to max entries; *n = the number of
+   shapes tried, 0 before any autotune).
    Results do not depend on the shapes.  No counterpart in the reference
    (its launches are fixed 16x16 thread blocks). */
 int rmhd2d_set_tile_shape(rmhd2d_solver *s, int shape);

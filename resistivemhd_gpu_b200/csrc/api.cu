@@ -57,7 +57,6 @@ struct rmhd2d_solver {
     CUtensorMap mapA[NSHAPE_ALL]{}, mapB[NSHAPE_ALL]{}, mapE1[NSHAPE_ALL]{}, mapE2[NSHAPE_ALL]{};
     int shape = 0;                       // tile shape of stage 1
     int shape2 = 0;                      // tile shape of stage 2
-    int own[2] = {-1, -1};               // shape the library picked for a stage (default_shapes, autotune), or -1
     void *batch = nullptr;               // owning batch, if any
     int parity = 0;
     bool has_state = false;
@@ -241,12 +240,8 @@ BatchLauncher batch_launcher(int precision)
     }
 }
 
-// The tile shape a stage runs: the library's own choice until the caller sets
-// one.
-int stage_plan(const rmhd2d_solver *s, int stage)
-{
-    return s->own[stage - 1] >= 0 ? s->own[stage - 1] : stage == 1 ? s->shape : s->shape2;
-}
+// The tile shape a stage runs.
+int stage_plan(const rmhd2d_solver *s, int stage) { return stage == 1 ? s->shape : s->shape2; }
 
 // Whether a grid's 4 x 16 tiles all run at once, two per SM.  Then a stage
 // lasts one block's latency, and a block of one interface per thread is the
@@ -262,15 +257,17 @@ bool small_grid(const Grid &g)
 // The shapes a solver starts with.  Large grids take what the autotuner finds
 // on them: three CTAs per SM win from about 2^18 cells (512 x 512, per step:
 // exact 117.2 -> 111.7 us, fast 84.1 -> 80.2, FP32-bulk 69.6 -> 62.5; 601 x
-// 347 and 384 x 384 are level), below that shape 0.
+// 347 and 384 x 384 are level), below that shape 0.  CT-Contact does not run
+// the tiled stage kernels.
 void default_shapes(rmhd2d_solver *s)
 {
     const Grid &g = s->g;
+    if (s->contact) return;
     if (small_grid(g)) {
-        s->own[0] = s->own[1] = SHAPE_SMALL;
+        s->shape = s->shape2 = SHAPE_SMALL;
     } else if ((long long)(g.nx - 2 * HALO) * (g.ny - 2 * HALO) >= 1LL << 18) {
-        s->own[0] = 4;
-        s->own[1] = s->cfg.precision == RMHD2D_FP32_BULK ? 4 : 5;
+        s->shape = 4;
+        s->shape2 = s->cfg.precision == RMHD2D_FP32_BULK ? 4 : 5;
     }
 }
 
@@ -931,14 +928,13 @@ int rmhd2d_load(rmhd2d_solver *s, const char *path)
 int rmhd2d_set_stage_shapes(rmhd2d_solver *s, int shape1, int shape2)
 {
     if (!s) return fail(s, RMHD2D_ERR_INVALID, "null solver");
-    if (shape1 < 0 || shape1 >= NSHAPE || shape2 < 0 || shape2 >= NSHAPE)
+    if (shape1 < 0 || shape1 >= NSHAPE_ALL || shape2 < 0 || shape2 >= NSHAPE_ALL)
         return fail(s, RMHD2D_ERR_INVALID, "unknown tile shape");
     CK(cudaSetDevice(s->device));
     CK(cudaStreamSynchronize(s->stream));
     destroy_graphs(s);
     s->shape = shape1;
     s->shape2 = shape2;
-    s->own[0] = s->own[1] = -1;
     return RMHD2D_OK;
 }
 
@@ -1030,14 +1026,11 @@ int rmhd2d_autotune(rmhd2d_solver *s, int trial_steps, int *best_shape)
     // Each stage's launch is timed by itself (the two stages read and write
     // different tiles and buffers), so the fastest shape is picked per stage:
     // the median over trial steps of each stage's CUDA-event time.
-    // On a small grid its own shape is tried too, and taken where it beats
-    // every public one.
-    s->tuning_ms.assign(2 * NSHAPE, 0.f);
-    const bool small = small_grid(s->g);
-    float small_ms[2] = {0.f, 0.f};
-    for (int sh = 0; sh < (small ? NSHAPE_ALL : NSHAPE) && rc == RMHD2D_OK; ++sh) {
-        rc = rmhd2d_set_stage_shapes(s, sh < NSHAPE ? sh : 0, sh < NSHAPE ? sh : 0);
-        if (sh == SHAPE_SMALL) s->own[0] = s->own[1] = SHAPE_SMALL;
+    // SHAPE_SMALL is tried where it is the start's shape.
+    const int nshape = small_grid(s->g) ? NSHAPE_ALL : NSHAPE;
+    s->tuning_ms.assign(2 * nshape, 0.f);
+    for (int sh = 0; sh < nshape && rc == RMHD2D_OK; ++sh) {
+        rc = rmhd2d_set_stage_shapes(s, sh, sh);
         if (!rc) rc = rmhd2d_run(s, 2);                          // warm-up
         std::vector<float> t1, t2;
         for (int k = 0; k < trial_steps && !rc; ++k) {
@@ -1049,22 +1042,19 @@ int rmhd2d_autotune(rmhd2d_solver *s, int trial_steps, int *best_shape)
         if (!rc) {
             std::sort(t1.begin(), t1.end());
             std::sort(t2.begin(), t2.end());
-            float *to = sh == SHAPE_SMALL ? small_ms : &s->tuning_ms[2 * sh];
-            to[0] = t1[t1.size() / 2];
-            to[1] = t2[t2.size() / 2];
+            s->tuning_ms[2 * sh] = t1[t1.size() / 2];
+            s->tuning_ms[2 * sh + 1] = t2[t2.size() / 2];
         }
     }
     const int rc2 = snapshot_restore(s, sn);
     if (rc) return rc;
     if (rc2) return rc2;
     int b1 = 0, b2 = 0;
-    for (int sh = 1; sh < NSHAPE; ++sh) {
+    for (int sh = 1; sh < nshape; ++sh) {
         if (s->tuning_ms[2 * sh] < s->tuning_ms[2 * b1]) b1 = sh;
         if (s->tuning_ms[2 * sh + 1] < s->tuning_ms[2 * b2 + 1]) b2 = sh;
     }
     rc = rmhd2d_set_stage_shapes(s, b1, b2);
-    if (small && small_ms[0] < s->tuning_ms[2 * b1]) s->own[0] = SHAPE_SMALL;
-    if (small && small_ms[1] < s->tuning_ms[2 * b2 + 1]) s->own[1] = SHAPE_SMALL;
     if (best_shape) *best_shape = b1;
     return rc;
 }

@@ -72,9 +72,10 @@ enum KernelError { KERR_NONE = 0, KERR_TMA_TIMEOUT = 1 };
 // Which is fastest for a variant and grid is the autotuners' question.
 constexpr int HALO = 3;
 constexpr int NSHAPE = 6;
-// SHAPE_SMALL, after them, is no public shape index: 4 x 16 cells (192 and 148
-// interfaces) for 192 threads, one interface each, for grids too small to
-// fill the SMs, where a stage takes as long as one block.
+// SHAPE_SMALL, after them, is for single runs only (batches have the shapes
+// before it): 4 x 16 cells (192 and 148 interfaces) for 192 threads, one
+// interface each, for grids too small to fill the SMs, where a stage takes as
+// long as one block.
 constexpr int SHAPE_SMALL = NSHAPE;
 constexpr int NSHAPE_ALL = NSHAPE + 1;
 constexpr int SM_COUNT = 148;

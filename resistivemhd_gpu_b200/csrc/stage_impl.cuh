@@ -916,7 +916,7 @@ struct LaunchBatch {
     cudaStream_t stream;
     template <int ST, int SH> void operator()() const
     {
-        if constexpr (SH < NSHAPE) {   // batches run the public shapes
+        if constexpr (SH < NSHAPE) {
             using T = Tile<ST, SH>;
             set_smem_attributes(stage_batch_kernel<ST, SH>, T::SMEM_BYTES, T::CTAS);
             const BatchRun *r = runs;

@@ -201,6 +201,7 @@ class Solver:
 
     @property
     def tile_shape(self) -> int:
+        """Tile shape of stage 1 as the next step runs it."""
         v = ctypes.c_int()
         self._ck(self._lib.rmhd2d_get_tile_shape(self._h, ctypes.byref(v)))
         return v.value
@@ -221,6 +222,7 @@ class Solver:
 
     @property
     def stage_shapes(self) -> tuple[int, int]:
+        """Tile shapes of stages 1 and 2 as the next step runs them."""
         a, b = ctypes.c_int(), ctypes.c_int()
         self._ck(self._lib.rmhd2d_get_stage_shapes(self._h, ctypes.byref(a), ctypes.byref(b)))
         return a.value, b.value
