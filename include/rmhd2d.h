@@ -210,7 +210,8 @@ int rmhd2d_write_snapshot(const char *path, const double *host_state, int nx, in
    threads, 3 CTAs per SM; 6: 4x16 / 4x16 with 192 threads, one interface
    each, 2 CTAs per SM (for grids too small to fill the SMs).
    A solver starts with shape 6 while the grid has at most 296 such tiles
-   (two per SM), with 4 and 5 (FP32-bulk: 4 and 4) from 2^18 interior cells,
+   (two per SM), with 4 and 5 (FP32-bulk, and beyond 458745 interior cells
+   along x: 4 and 4) from 2^18 interior cells,
    and with shape 0 between.  Each stage has its own shape:
    rmhd2d_set_tile_shape sets both, rmhd2d_set_stage_shapes each,
    rmhd2d_get_tile_shape returns stage 1's, rmhd2d_get_stage_shapes both, as

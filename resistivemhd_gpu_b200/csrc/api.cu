@@ -257,8 +257,10 @@ bool small_grid(const Grid &g)
 // The shapes a solver starts with.  Large grids take what the autotuner finds
 // on them: three CTAs per SM win from about 2^18 cells (512 x 512, per step:
 // exact 117.2 -> 111.7 us, fast 84.1 -> 80.2, FP32-bulk 69.6 -> 62.5; 601 x
-// 347 and 384 x 384 are level), below that shape 0.  CT-Contact does not run
-// the tiled stage kernels.
+// 347 and 384 x 384 are level), below that shape 0.  A launch has at most 65535
+// rows of tiles (gridDim.y): where shape 5's seven cells per row are too few,
+// stage 2 takes shape 4, whose eight are as many as shape 0's.  CT-Contact does
+// not run the tiled stage kernels.
 void default_shapes(rmhd2d_solver *s)
 {
     const Grid &g = s->g;
@@ -267,7 +269,7 @@ void default_shapes(rmhd2d_solver *s)
         s->shape = s->shape2 = SHAPE_SMALL;
     } else if ((long long)(g.nx - 2 * HALO) * (g.ny - 2 * HALO) >= 1LL << 18) {
         s->shape = 4;
-        s->shape2 = s->cfg.precision == RMHD2D_FP32_BULK ? 4 : 5;
+        s->shape2 = s->cfg.precision == RMHD2D_FP32_BULK || g.nx - 2 * HALO > 65535 * stage_ti(2, 5) ? 4 : 5;
     }
 }
 
