@@ -6,6 +6,7 @@
 #include "aux_kernels.h"
 #include "cell_block.cuh"
 #include "physics.cuh"
+#include "stage.cuh"
 
 namespace rmhd2d {
 
@@ -330,7 +331,7 @@ boundary_kernel(Grid g, double *s, const double *row2, Control *ctl, int slot, C
     if (live) {
         const double r = cfl_rate(sv[RHO][lane], sv[MX][lane], sv[MY][lane], sv[MZ][lane], sv[BXF][lane],
                                   sv[BYF][lane], sv[BZF][lane], sv[EN][lane], g.gamma, g.dx, g.dy);
-        bits = rate_bits(r);
+        if (!(BX == BC_PERIODIC && BY == BC_PERIODIC)) bits = rate_bits(r);   // (all_periodic)
         nan_e = sv[EN][lane] != sv[EN][lane];
         c0 = (i == 0 && j == 0 && r != r);
     }
@@ -358,7 +359,7 @@ __global__ void boundary_batch_kernel(const BatchRun *runs, int which, int slot)
     const Grid &g = r.g;
     const long long nghost = 6LL * g.ny + 6LL * (g.nx - 6);
     const long long first = (long long)blockIdx.x * blockDim.x;
-    if (first >= nghost) return;   // whole warp-aligned block beyond this run
+    if (first >= nghost || wraps(g)) return;   // whole warp-aligned block beyond this run, or nothing left to fill
     const long long t = first + threadIdx.x;
     unsigned long long bits = 0ull;
     int nan_e = 0;
@@ -483,7 +484,7 @@ __global__ void slab_origin_column_kernel(Grid g, double *s, Control *ctl, int s
     if (g.bc_y == BC_SYMMETRIC) s[BYF * P + k] = s[BYF * P + at(g, 0, j < 3 ? 3 : g.ny - 4)];
     const double r = cfl_rate(s[RHO * P + k], s[MX * P + k], s[MY * P + k], s[MZ * P + k], s[BXF * P + k],
                               s[BYF * P + k], s[BZF * P + k], s[EN * P + k], g.gamma, g.dx, g.dy);
-    const unsigned long long b = rate_bits(r);
+    const unsigned long long b = all_periodic(g) ? 0ull : rate_bits(r);
     if (b) atomicMax(&ctl->amax[slot], b);
     if (j == 0 && r != r) ctl->first_nan[slot] = 1;
 }

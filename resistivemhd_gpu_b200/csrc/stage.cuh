@@ -49,11 +49,18 @@ struct StageArgs {
     Control *mirror;     // stage 2 with wrap, or nullptr: the launch leaves the control block there (host memory)
 };
 
-// Whether the stage kernels write a grid's ghost cells themselves.
-__host__ __device__ __forceinline__ bool wraps(const Grid &g)
+// Whether every ghost cell of the domain is the image of an interior cell.
+// The stage-2 kernel has then reduced all its CFL rates, and a ghost fill adds
+// none: its rates are uncontracted, and the contracted variants' dt would
+// otherwise depend on whether a fill runs -- in a batch on the other runs'
+// walls, in a decomposed domain on the decomposition.
+__host__ __device__ __forceinline__ bool all_periodic(const Grid &g)
 {
-    return g.bc_x == BC_PERIODIC && g.bc_y == BC_PERIODIC && !g.x_halo;
+    return g.bc_x == BC_PERIODIC && g.bc_y == BC_PERIODIC;
 }
+
+// Whether the stage kernels write a grid's ghost cells themselves.
+__host__ __device__ __forceinline__ bool wraps(const Grid &g) { return all_periodic(g) && !g.x_halo; }
 
 // One set of launchers per variant (stage_exact.cu, stage_fast.cu, stage_bulk32.cu).
 // Sweep of the stage kernel's flux phase (true: x sweep), as a compile-time
