@@ -291,25 +291,18 @@ __device__ __forceinline__ void add_weighted_flux(double rho, double u, double v
 
 // HLLD flux through one interface: hlld.cu:256-432
 // (calculateHLLDParameterFunctor), hlld.cu:469-549 (setFluxFunctor) and
-// hlld.cu:35-107 (CalculateFluxFunctor), with the divisions of the policy
-// Div (MdDiv: shared correctly rounded reciprocals; IeeeDiv: plain division);
-// both give the reference's quotients bit for bit while Div::ok holds.
-// ygm1 is Div's reciprocal handle of gm - 1.
-//
-// ALL_CANDIDATES = true gives the bits of the reference's sum of all six
-// candidate fluxes with 0/1 indicator weights for every input, including
-// non-finite ones: it forms that sum unless exactly one candidate is selected
-// and all candidate values are bounded, where the selected flux alone has the
-// same bits.  ALL_CANDIDATES = false forms only the candidates whose
-// indicator is 1 and adds them in the reference's order, which gives the same
-// bits whenever all six candidates are finite.
-template <bool ALL_CANDIDATES, class Div>
-__device__ __forceinline__ void hlld_body(const Prim &L, const Prim &R, double gm, double EPS, double ygm1, Div &dv,
-                                          double f[8])
+// hlld.cu:35-107 (CalculateFluxFunctor), the reference's arithmetic in full
+// with IEEE division: the rare path of hlld_flux_sel.  It gives the bits of
+// the reference's sum of all six candidate fluxes with 0/1 indicator weights
+// for every input, including non-finite ones: it forms that sum unless exactly
+// one candidate is selected and all candidate values are bounded, where the
+// selected flux alone has the same bits.
+__device__ __forceinline__ void hlld_flux_ieee(const Prim &L, const Prim &R, double gm, double EPS, double f[8])
 {
+    IeeeDiv dv;
     const double rhoL = L.rho, uL = L.u, vL = L.v, wL = L.w, bXL = L.bX, bYL = L.bY, bZL = L.bZ, pL = L.p;
     const double rhoR = R.rho, uR = R.u, vR = R.v, wR = R.w, bXR = R.bX, bYR = R.bY, bZR = R.bZ, pR = R.p;
-    const double gm1 = gm - 1.0;
+    const double gm1 = gm - 1.0, ygm1 = dv.recip(gm1);
 
     const double eL = dv.div(pL, gm1, ygm1)
                     + 0.5 * rhoL * (uL * uL + vL * vL + wL * wL)
@@ -401,94 +394,52 @@ __device__ __forceinline__ void hlld_body(const Prim &L, const Prim &R, double g
 
 #pragma unroll
     for (int n = 0; n < 8; ++n) f[n] = 0.0;
-    if (ALL_CANDIDATES) {
-        // The weighted sum adds F * 0 = +-0 for every unselected candidate
-        // whose flux is finite, which leaves the selected candidate's flux
-        // bit for bit.  A flux component is a product of at most three of
-        // the candidate's values plus a few such products, so it is finite
-        // whenever every value is below 1e75 in magnitude; the sum of
-        // magnitudes below is NaN or infinite, and fails the test, as soon
-        // as one value is.  Then, with exactly one region selected, only
-        // that candidate is formed; otherwise all six are.
-        const int nsel = (int)bOL + (int)bML + (int)bIL + (int)bOR + (int)bMR + (int)bIR;
-        const double mag = fabs(rhoL) + fabs(uL) + fabs(vL) + fabs(wL) + fabs(bXL) + fabs(bYL) + fabs(bZL)
-                         + fabs(eL) + fabs(pTL) + fabs(rhoR) + fabs(uR) + fabs(vR) + fabs(wR) + fabs(bXR)
-                         + fabs(bYR) + fabs(bZR) + fabs(eR) + fabs(pTR) + fabs(rho1L) + fabs(rho1R) + fabs(SM)
-                         + fabs(pT1) + fabs(v1L) + fabs(w1L) + fabs(bY1L) + fabs(bZ1L) + fabs(e1L) + fabs(v1R)
-                         + fabs(w1R) + fabs(bY1R) + fabs(bZ1R) + fabs(e1R) + fabs(v2) + fabs(w2) + fabs(bY2)
-                         + fabs(bZ2) + fabs(e2L) + fabs(e2R);
-        if (nsel == 1 && mag < 1e75) {
-            const bool lft = bOL | bML | bIL;
-            const bool outer = bOL | bOR, inner = bIL | bIR;
-            const double rho = bOL ? rhoL : (bOR ? rhoR : (lft ? rho1L : rho1R));
-            const double u = bOL ? uL : (bOR ? uR : SM);
-            const double v = outer ? (bOL ? vL : vR) : (inner ? v2 : (bML ? v1L : v1R));
-            const double w = outer ? (bOL ? wL : wR) : (inner ? w2 : (bML ? w1L : w1R));
-            const double bx = lft ? bXL : bXR;
-            const double by = outer ? (bOL ? bYL : bYR) : (inner ? bY2 : (bML ? bY1L : bY1R));
-            const double bz = outer ? (bOL ? bZL : bZR) : (inner ? bZ2 : (bML ? bZ1L : bZ1R));
-            const double e = bOL ? eL : (bOR ? eR : (bML ? e1L : (bIL ? e2L : (bMR ? e1R : e2R))));
-            const double pT = bOL ? pTL : (bOR ? pTR : pT1);
-            add_one_flux(rho, u, v, w, bx, by, bz, e, pT, f);
-            return;
-        }
-        // rho2L = rho1L, rho2R = rho1R, pT2 = pT1 (hlld.cu:360-378).
-        add_weighted_flux(rhoL, uL, vL, wL, bXL, bYL, bZL, eL, pTL, (double)bOL, f);
-        add_weighted_flux(rho1L, u1L, v1L, w1L, bXL, bY1L, bZ1L, e1L, pT1, (double)bML, f);
-        add_weighted_flux(rho1L, u2, v2, w2, bXL, bY2, bZ2, e2L, pT1, (double)bIL, f);
-        add_weighted_flux(rhoR, uR, vR, wR, bXR, bYR, bZR, eR, pTR, (double)bOR, f);
-        add_weighted_flux(rho1R, u1R, v1R, w1R, bXR, bY1R, bZ1R, e1R, pT1, (double)bMR, f);
-        add_weighted_flux(rho1R, u2, v2, w2, bXR, bY2, bZ2, e2R, pT1, (double)bIR, f);
-    } else {
-        if (bOL) add_one_flux(rhoL, uL, vL, wL, bXL, bYL, bZL, eL, pTL, f);
-        if (bML) add_one_flux(rho1L, u1L, v1L, w1L, bXL, bY1L, bZ1L, e1L, pT1, f);
-        if (bIL) add_one_flux(rho1L, u2, v2, w2, bXL, bY2, bZ2, e2L, pT1, f);
-        if (bOR) add_one_flux(rhoR, uR, vR, wR, bXR, bYR, bZR, eR, pTR, f);
-        if (bMR) add_one_flux(rho1R, u1R, v1R, w1R, bXR, bY1R, bZ1R, e1R, pT1, f);
-        if (bIR) add_one_flux(rho1R, u2, v2, w2, bXR, bY2, bZ2, e2R, pT1, f);
+    // The weighted sum adds F * 0 = +-0 for every unselected candidate
+    // whose flux is finite, which leaves the selected candidate's flux
+    // bit for bit.  A flux component is a product of at most three of
+    // the candidate's values plus a few such products, so it is finite
+    // whenever every value is below 1e75 in magnitude; the sum of
+    // magnitudes below is NaN or infinite, and fails the test, as soon
+    // as one value is.  Then, with exactly one region selected, only
+    // that candidate is formed; otherwise all six are.
+    const int nsel = (int)bOL + (int)bML + (int)bIL + (int)bOR + (int)bMR + (int)bIR;
+    const double mag = fabs(rhoL) + fabs(uL) + fabs(vL) + fabs(wL) + fabs(bXL) + fabs(bYL) + fabs(bZL)
+                     + fabs(eL) + fabs(pTL) + fabs(rhoR) + fabs(uR) + fabs(vR) + fabs(wR) + fabs(bXR)
+                     + fabs(bYR) + fabs(bZR) + fabs(eR) + fabs(pTR) + fabs(rho1L) + fabs(rho1R) + fabs(SM)
+                     + fabs(pT1) + fabs(v1L) + fabs(w1L) + fabs(bY1L) + fabs(bZ1L) + fabs(e1L) + fabs(v1R)
+                     + fabs(w1R) + fabs(bY1R) + fabs(bZ1R) + fabs(e1R) + fabs(v2) + fabs(w2) + fabs(bY2)
+                     + fabs(bZ2) + fabs(e2L) + fabs(e2R);
+    if (nsel == 1 && mag < 1e75) {
+        const bool lft = bOL | bML | bIL;
+        const bool outer = bOL | bOR, inner = bIL | bIR;
+        const double rho = bOL ? rhoL : (bOR ? rhoR : (lft ? rho1L : rho1R));
+        const double u = bOL ? uL : (bOR ? uR : SM);
+        const double v = outer ? (bOL ? vL : vR) : (inner ? v2 : (bML ? v1L : v1R));
+        const double w = outer ? (bOL ? wL : wR) : (inner ? w2 : (bML ? w1L : w1R));
+        const double bx = lft ? bXL : bXR;
+        const double by = outer ? (bOL ? bYL : bYR) : (inner ? bY2 : (bML ? bY1L : bY1R));
+        const double bz = outer ? (bOL ? bZL : bZR) : (inner ? bZ2 : (bML ? bZ1L : bZ1R));
+        const double e = bOL ? eL : (bOR ? eR : (bML ? e1L : (bIL ? e2L : (bMR ? e1R : e2R))));
+        const double pT = bOL ? pTL : (bOR ? pTR : pT1);
+        add_one_flux(rho, u, v, w, bx, by, bz, e, pT, f);
+        return;
     }
-}
-
-// The exact HLLD flux: shared correctly rounded reciprocals, repeated with
-// IEEE division where the guard of MdDiv fails (non-finite, huge or tiny
-// operands).  ygm1 = rcp_rn_md(gm - 1), gm1_ok = MdDiv's guard on it.
-template <bool ALL_CANDIDATES>
-__device__ __forceinline__ void hlld_flux(const Prim &L, const Prim &R, double gm, double EPS, double ygm1,
-                                          bool gm1_ok, double f[8])
-{
-    MdDiv md;
-    md.ok = gm1_ok;
-    hlld_body<ALL_CANDIDATES>(L, R, gm, EPS, ygm1, md, f);
-    if (!md.ok) {
-        IeeeDiv id;
-        hlld_body<ALL_CANDIDATES>(L, R, gm, EPS, gm - 1.0, id, f);
-    }
-}
-
-// The same, forming the reciprocal of gm - 1 itself.
-template <bool ALL_CANDIDATES>
-__device__ __forceinline__ void hlld_flux(const Prim &L, const Prim &R, double gm, double EPS, double f[8])
-{
-    MdDiv g1;
-    const double ygm1 = g1.recip(gm - 1.0);
-    hlld_flux<ALL_CANDIDATES>(L, R, gm, EPS, ygm1, g1.ok, f);
-}
-
-// The reference's arithmetic in full: IEEE division and all six candidates
-// weighted, for every input.  The rare path of hlld_flux_sel.
-__device__ __forceinline__ void hlld_flux_ieee(const Prim &L, const Prim &R, double gm, double EPS, double f[8])
-{
-    IeeeDiv id;
-    hlld_body<true>(L, R, gm, EPS, gm - 1.0, id, f);
+    // rho2L = rho1L, rho2R = rho1R, pT2 = pT1 (hlld.cu:360-378).
+    add_weighted_flux(rhoL, uL, vL, wL, bXL, bYL, bZL, eL, pTL, (double)bOL, f);
+    add_weighted_flux(rho1L, u1L, v1L, w1L, bXL, bY1L, bZ1L, e1L, pT1, (double)bML, f);
+    add_weighted_flux(rho1L, u2, v2, w2, bXL, bY2, bZ2, e2L, pT1, (double)bIL, f);
+    add_weighted_flux(rhoR, uR, vR, wR, bXR, bYR, bZR, eR, pTR, (double)bOR, f);
+    add_weighted_flux(rho1R, u1R, v1R, w1R, bXR, bY1R, bZ1R, e1R, pT1, (double)bMR, f);
+    add_weighted_flux(rho1R, u2, v2, w2, bXR, bY2, bZ2, e2R, pT1, (double)bIR, f);
 }
 
 // The exact HLLD flux with the candidate picked as the fan is built.  Every
-// value is the same expression as in hlld_body, so the bits are those of
-// hlld_flux<true>; only what stays live differs.  hlld_body keeps all six
-// candidate states (38 values) live until the region flags are known and
-// then selects; here each candidate is taken into the nine `c*` values as
-// soon as its own flag is known, so the left and right input states die
-// after the star states.  Where the shortcut's conditions fail it returns
+// value is the same expression as in hlld_flux_ieee, with the divisions of
+// MdDivFlux, so the bits are the same; only what stays live differs.
+// hlld_flux_ieee keeps all six candidate states (38 values) live until the
+// region flags are known and then selects; here each candidate is taken into
+// the nine `c*` values as soon as its own flag is known, so the left and right
+// input states die after the star states.  Where the shortcut's conditions fail it returns
 // false with f unwritten, and the caller forms the interface with
 // hlld_flux_ieee, away from its common path (the stage kernel's flux phase
 // does that after its loop, for the interfaces that asked, so the rare path
@@ -637,7 +588,7 @@ __device__ __forceinline__ bool hlld_flux_sel(const Prim &L, const Prim &R, doub
 }
 
 // HLLD flux of the fast variant: the same wave-speed estimates, star and
-// double-star states and candidate selection as hlld_flux (hlld.cu:256-565),
+// double-star states and candidate selection as hlld_flux_sel (hlld.cu:256-565),
 // rearranged for the FP64 pipe.  It differs from the exact form by rounding
 // only: one correctly rounded reciprocal per distinct denominator (8 instead
 // of 28 divisions), squared sound/Alfven speeds used directly (the reference
