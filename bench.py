@@ -220,7 +220,11 @@ def reference_arm(args, rank: int) -> None:
         return
     setup, label = workload(args.workload)
     threads = os.cpu_count() or 1
-    info = run_reference_binary("cpu", setup, args.warmup, args.steps, threads)
+    try:
+        info = run_reference_binary("cpu", setup, args.warmup, args.steps, threads)
+    except FileNotFoundError as e:   # no reference sources to build it from
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     secs = info["seconds"]
     value = setup.interior_cells * args.steps / secs
     line = {
