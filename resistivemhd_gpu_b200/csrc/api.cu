@@ -1569,6 +1569,7 @@ int rmhd2d_slab_stage(rmhd2d_solver *s, int stage)
     a.row2 = s->g.bc_x == BC_SYMMETRIC ? s->row2 : nullptr;
     a.ctl = s->ctl;
     a.parity = s->parity;
+    a.wrap = wraps(s->g);
     if (stage == 1) {
         a.src = s->A;
         a.un = s->A;
@@ -1596,9 +1597,9 @@ int rmhd2d_slab_fill(rmhd2d_solver *s, int which)
         if (s->g.bc_x == BC_SYMMETRIC) launch_snapshot_row2(s->g, s->A, s->row2, s->stream);
         launch_boundary(s->g, s->A, s->row2, nullptr, 0, s->stream);
     } else if (which == 1) {
-        launch_boundary(s->g, s->B, s->row2, nullptr, 0, s->stream);
+        if (!wraps(s->g)) launch_boundary(s->g, s->B, s->row2, nullptr, 0, s->stream);
     } else {
-        launch_boundary(s->g, s->A, s->row2, s->ctl, s->parity ^ 1, s->stream);
+        if (!wraps(s->g)) launch_boundary(s->g, s->A, s->row2, s->ctl, s->parity ^ 1, s->stream);
         s->parity ^= 1;
         s->steps += 1;
     }

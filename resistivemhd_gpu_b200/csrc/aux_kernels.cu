@@ -331,7 +331,7 @@ boundary_kernel(Grid g, double *s, const double *row2, Control *ctl, int slot, C
     if (live) {
         const double r = cfl_rate(sv[RHO][lane], sv[MX][lane], sv[MY][lane], sv[MZ][lane], sv[BXF][lane],
                                   sv[BYF][lane], sv[BZF][lane], sv[EN][lane], g.gamma, g.dx, g.dy);
-        if (!(BX == BC_PERIODIC && BY == BC_PERIODIC)) bits = rate_bits(r);   // (all_periodic)
+        if (!(BX == BC_PERIODIC && BY == BC_PERIODIC && g.x_halo)) bits = rate_bits(r);   // (all_periodic)
         nan_e = sv[EN][lane] != sv[EN][lane];
         c0 = (i == 0 && j == 0 && r != r);
     }

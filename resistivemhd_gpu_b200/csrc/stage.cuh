@@ -50,10 +50,10 @@ struct StageArgs {
 };
 
 // Whether every ghost cell of the domain is the image of an interior cell.
-// The stage-2 kernel has then reduced all its CFL rates, and a ghost fill adds
-// none: its rates are uncontracted, and the contracted variants' dt would
-// otherwise depend on whether a fill runs -- in a batch on the other runs'
-// walls, in a decomposed domain on the decomposition.
+// The stage-2 kernel has then reduced all its CFL rates, and the ghost fill of
+// a slab adds none: its rates are uncontracted, and the contracted variants'
+// dt would otherwise depend on whether a fill runs.  For the same reason a
+// batch's fill leaves out the runs that need none.
 __host__ __device__ __forceinline__ bool all_periodic(const Grid &g)
 {
     return g.bc_x == BC_PERIODIC && g.bc_y == BC_PERIODIC;

@@ -2,6 +2,8 @@
 stepped: by itself, in a batch beside runs with walls, or decomposed into
 slabs.  The contracted variants would otherwise mix in the ghost fill's
 uncontracted rates where one runs, and differ in the last bit."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -53,6 +55,44 @@ def _check_slabs(precision, torch_device):
                     whole.step()
                     g.step()
                 assert np.array_equal(g.get_state(), whole.get_state()), (seed, parts)
+
+
+def _check_slab_without_halos(lib, precision):
+    """The whole domain as one slab with no halo columns, through the C ABI."""
+    from resistivemhd_gpu_b200 import Solver, setups
+
+    D = ctypes.POINTER(ctypes.c_double)
+    for seed in SEEDS:
+        s = setups.random_smooth_state(24, 20, seed=seed, bc="periodic")
+        with Solver.from_setup(s, precision=precision) as whole:
+            whole.run(4)
+            want = whole.get_state()
+        cfg = Solver.make_config(s.nx, s.ny, s.dx, s.dy, gamma=s.gamma, cfl=s.cfl, eps=s.eps, eta=s.eta, bc=s.bc,
+                                 precision=precision)
+        h, st = ctypes.c_void_p(), np.ascontiguousarray(s.state)
+        assert lib.rmhd2d_create_slab(ctypes.byref(cfg), 4, ctypes.byref(h)) == 0
+        try:
+            assert lib.rmhd2d_set_state(h, st.ctypes.data_as(D), 1) == 0
+            for _ in range(4):
+                for k in (1, 2):
+                    assert lib.rmhd2d_slab_stage(h, k) == 0
+                    assert lib.rmhd2d_slab_fill(h, k) == 0
+            got = np.empty_like(st)
+            assert lib.rmhd2d_get_state(h, got.ctypes.data_as(D)) == 0
+        finally:
+            lib.rmhd2d_destroy(h)
+        assert np.array_equal(got, want), seed
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_slab_without_halos_on_the_host_build(on_host, host_abi, precision):
+    _check_slab_without_halos(host_abi, precision)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_slab_without_halos(gpu, precision):
+    _check_slab_without_halos(gpu, precision)
 
 
 @pytest.mark.parametrize("precision", PRECISIONS)
