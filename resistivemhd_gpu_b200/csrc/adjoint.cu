@@ -259,7 +259,7 @@ __global__ void periodic_transpose_kernel(Grid g, double *Ub)
 // cleared by the launch after it.  Every value is loaded before the first
 // store: with one thread per line and all fields' read-modify-writes in a
 // row, each waited for the one before it (150 x 90: 27 + 18 us per transpose,
-// now 3.5 + 3.5).  The x pass at row 3 reads the lower wall face bY(c,2)
+// now 4.5 + 3.3 and 2.3 for the last clear).  The x pass at row 3 reads the lower wall face bY(c,2)
 // before the y pass replaces it -- in the step, the stage-1 CT result (row2)
 // -- so the x transpose leaves that adjoint in the ghost entry (c,2) of the
 // interior columns, where the stage-1 reverse takes it as the CT'd face's.

@@ -1283,7 +1283,7 @@ int rmhd2d_batch_set_launch(rmhd2d_batch *b, int shape, int ctas_per_sm)
 {
     if (!b) return bfail(b, RMHD2D_ERR_INVALID, "null batch");
     if (shape < 0 || shape >= NSHAPE || ctas_per_sm < 1 || ctas_per_sm > shape_max_ctas(shape))
-        return bfail(b, RMHD2D_ERR_INVALID, "tile shape must be 0..2 and CTAs per SM 1..2 (1 for shape 2)");
+        return bfail(b, RMHD2D_ERR_INVALID, "tile shape must be 0..5 with 1 up to the shape's CTAs per SM");
     b->shape = shape;
     b->ctas_per_sm = ctas_per_sm;
     b->dirty = true;

@@ -557,7 +557,9 @@ void launch_snapshot_row2(const Grid &g, const double *s, double *row2, cudaStre
 
 void launch_rate(const Grid &g, const double *s, Control *ctl, int slot, int set_crash, cudaStream_t st)
 {
-    const unsigned groups = CellBlock<RATE_ROWS>::blocks(g), most = 148u * 8u;   // all resident at once
+    // at most two rounds of the four blocks per SM that 56 registers allow; from
+    // there on a block walks several groups
+    const unsigned groups = CellBlock<RATE_ROWS>::blocks(g), most = 2u * 4u * SM_COUNT;
     rate_kernel<<<groups < most ? groups : most, CellBlock<RATE_ROWS>::THREADS, 0, st>>>(g, s, ctl, slot, set_crash);
 }
 

@@ -75,8 +75,9 @@ __device__ __forceinline__ double by_s(const Grid &g, const double *U, int i, in
 // reference's quotients bit for bit.  The flux takes its common path in the
 // loop and the declined interfaces after it, as the stage kernels do: it then
 // fits 80 registers and three CTAs per SM (24 warps; FP64-issue bound).  Harris
-// 2048 x 1024: 382 us a launch at two CTAs with every candidate kept, 316 now;
-// at two CTAs the step took 1235 us, at three 1176.
+// 2048 x 1024: 384 us a launch at two CTAs with every candidate kept, 315 now.
+// With the common path the step took 1235 us at two CTAs and 1176 at three
+// (1133 now, with the planes and blocks of the other kernels).
 constexpr int CT_TI = 16, CT_TJ = 32, CT_THREADS = 256, CT_CTAS = 3;
 constexpr int CT_SI = CT_TI + 3, CT_SJ = CT_TJ + 3, CT_SC = CT_SI * CT_SJ;
 constexpr int CT_JI = CT_TI + 1, CT_JJ = CT_TJ + 1, CT_JC = CT_JI * CT_JJ;

@@ -173,7 +173,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t phase)
 // Writes a cell's new values v, and under periodic walls (wrap) its ghost
 // images (boundary.cu:4-141): ghost c < 3 holds cell c + n - 6, ghost c >= n - 3
 // cell c - (n - 6).  This spares the step's two ghost-fill launches, about 4 us
-// each (exact, 128 x 128: 22.6 -> 17.4 us per step).
+// each (exact, 128 x 128: 22.6 -> 16.5 us per step).
 __device__ __forceinline__ void store_cell(const Grid &g, double *dst, int i, int j, bool wrap, const double v[NFIELD])
 {
     double *p = dst + (long long)i * g.pitch + j;
