@@ -47,6 +47,18 @@ def tangent():
 
 
 @pytest.fixture(scope="session")
+def shared_host_abi(tmp_path_factory):
+    """(library, its folder of objects): the host build of the whole C ABI
+    (tests/host_build.py), built once for the session."""
+    from host_build import build_host_abi, has_fma
+
+    if not has_fma():
+        pytest.skip("the host has no fused multiply-add to model the device build with")
+    d = tmp_path_factory.mktemp("sharedabi")
+    return build_host_abi(d), d
+
+
+@pytest.fixture(scope="session")
 def gpu(request, tmp_path_factory):
     """Skips nothing: a GPU test run without a usable B200 is a failure.
 

@@ -7,7 +7,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from host_build import EMU, HERE, build_host_abi, has_fma, link
+from host_build import EMU, HERE, link
 
 CAPTURE_HOST = """
 #include "cuda_runtime.h"
@@ -149,11 +149,8 @@ def _queries_follow_a_replay(lib, graphs, bc, work):
 
 
 @pytest.fixture(scope="module")
-def host_abi(tmp_path_factory):
-    if not has_fma():
-        pytest.skip("the host has no fused multiply-add to model the device build with")
-    d = tmp_path_factory.mktemp("capture")
-    build_host_abi(d)
+def host_abi(shared_host_abi):
+    _, d = shared_host_abi
     src = d / "capture_host.cpp"
     src.write_text(CAPTURE_HOST)
     lib = link(d, sorted(str(o) for o in d.glob("*.o")), [HERE / "host_tma.cpp", src], "librmhd2d_capture.so", (EMU,))

@@ -4,18 +4,14 @@ Setting the shapes that were read changes nothing."""
 import numpy as np
 import pytest
 
-from host_build import build_host_abi, has_fma
-
 LARGE = {"fp64_exact": (4, 5), "fp64_fast": (4, 5), "fp32_bulk": (4, 4)}
 
 
 @pytest.fixture
-def on_host(tmp_path_factory, monkeypatch):
-    if not has_fma():
-        pytest.skip("the host has no fused multiply-add to model the device build with")
+def on_host(shared_host_abi, monkeypatch):
     from resistivemhd_gpu_b200 import _lib
 
-    monkeypatch.setattr(_lib, "_lib", build_host_abi(tmp_path_factory.mktemp("shapes")))
+    monkeypatch.setattr(_lib, "_lib", shared_host_abi[0])
 
 
 def _solver(n, m, precision="fp64_exact", ct="stage1"):

@@ -3,8 +3,6 @@ of tiles than a launch takes (gridDim.y, 65535)."""
 import numpy as np
 import pytest
 
-from host_build import build_host_abi, has_fma
-
 LIMIT = 65535
 
 
@@ -15,12 +13,10 @@ def _start_shapes(n):
         return sol.stage_shapes
 
 
-def test_start_shapes_launch_on_the_host_build(tmp_path, monkeypatch):
-    if not has_fma():
-        pytest.skip("the host has no fused multiply-add to model the device build with")
+def test_start_shapes_launch_on_the_host_build(shared_host_abi, monkeypatch):
     from resistivemhd_gpu_b200 import _lib
 
-    monkeypatch.setattr(_lib, "_lib", build_host_abi(tmp_path))
+    monkeypatch.setattr(_lib, "_lib", shared_host_abi[0])
     assert _start_shapes(7 * LIMIT) == (4, 5)
     assert _start_shapes(7 * LIMIT + 1) == (4, 4)
 
